@@ -197,6 +197,12 @@ static void apply_tuning_file(fr_handle *h)
   h->tuned = true;
 }
 
+// The item split of the handle's launch shape (after its grid and groups are settled).
+static frb::ItemSplit handle_split(const fr_handle *h)
+{
+  return frb::item_split(h->launch.item_capacity, h->grid * frb::insert_groups(h->cfg), h->cfg);
+}
+
 int frb::batch_device_status(const fr_handle *h) { return h && h->host_status ? h->host_status[0] : FR_E_INVALID; }
 
 static cudaEvent_t next_event(fr_handle *h, int &idx)
@@ -422,7 +428,7 @@ int fr_init(fr_handle *h, const fr_dims *d, const fr_settings *s)
   cfg.groups = h->launch.groups;
   h->launch.groups = frb::insert_groups(cfg);
 
-  if (h->launch.item_capacity <= 0) h->launch.item_capacity = 512;
+  if (h->launch.item_capacity <= 0) h->launch.item_capacity = frb::kItemCapacity;
   h->launch.brick = 16;
   size_t smem = frb::insert_smem_bytes(cfg, int(d->table_elems));
   int occ = 0;
@@ -443,7 +449,7 @@ int fr_init(fr_handle *h, const fr_dims *d, const fr_settings *s)
   h->chunk_cap = std::min<int64_t>(int64_t(d->n_spaces), 65536);
   while (h->chunk_cap > 1 && h->chunk_cap * perSpace > (int64_t(1) << 30)) h->chunk_cap /= 2;
   const int64_t listCap = h->chunk_cap * perSpace;
-  const int64_t itemsCap = listCap / h->launch.item_capacity + g.n_bricks + 1;
+  const int64_t itemsCap = listCap / h->launch.item_capacity + handle_split(h).want + g.n_bricks + 1;
 
   // Brick visiting order: nearest to the volume centre first (they carry the most slabs).
   std::vector<int> order(g.n_bricks);
@@ -718,7 +724,7 @@ int fr_execute(fr_handle *h, const void *fft, const float *scales, uint64_t nPro
     int e0 = -1, e1 = -1, e2 = -1;
     if (h->profiling) FR_CUDA(cudaEventRecord(next_event(h, e0), h->stream));
     FR_CUDA(frb::launch_binning(h->geom, spaces + s0, n, int(nProj), h->cfg.fast, s.blob_radius, h->bb,
-      h->launch.item_capacity, h->stream));
+      handle_split(h), h->stream));
     FR_CUDA(cudaMemsetAsync(h->work_counter, 0, sizeof(int), h->stream));
     if (bandCopy && s0 == 0) FR_CUDA(cudaStreamWaitEvent(h->stream, h->band_join, 0));
     if (h->profiling) FR_CUDA(cudaEventRecord(next_event(h, e1), h->stream));
@@ -790,7 +796,7 @@ int fr_batch_init(fr_handle *h, const fr_batch_limits *lim, const fr_settings *s
   apply_tuning_file(h);
   cfg.groups = h->launch.groups;
   h->launch.groups = frb::insert_groups(cfg);
-  if (h->launch.item_capacity <= 0) h->launch.item_capacity = 512;
+  if (h->launch.item_capacity <= 0) h->launch.item_capacity = frb::kItemCapacity;
   h->launch.brick = 16;
   const size_t smem = frb::insert_smem_bytes(cfg, int(lim->table_elems));
   int occ = 0;
@@ -804,7 +810,7 @@ int fr_batch_init(fr_handle *h, const fr_batch_limits *lim, const fr_settings *s
   const int64_t listCap = int64_t(lim->max_spaces) * perSpace;
   if (listCap > (int64_t(1) << 31) - 1) return fail(FR_E_UNSUPPORTED, "batch limits exceed the list index range");
   const int64_t nb = int64_t(lim->max_bricks);
-  const int64_t itemsCap = listCap / h->launch.item_capacity + nb + 1;
+  const int64_t itemsCap = listCap / h->launch.item_capacity + handle_split(h).want + nb + 1;
   size_t off = 0;
   auto take = [&](size_t bytes) {
     size_t o = off;
@@ -881,7 +887,7 @@ static int enqueue_batch(fr_handle *h, int nJobs, int totalSpaces, int totalBric
   FR_CUDA(cudaEventRecord(h->band_join, h->band_stream));
   FR_CUDA(cudaMemsetAsync(h->bb.stats, 0, 4 * sizeof(unsigned long long), h->stream));
   FR_CUDA(frb::launch_batch_binning(h->d_jobs, nJobs, totalSpaces, totalBricks, totalGroups, h->cfg.fast,
-    s.blob_radius, h->bb, h->launch.item_capacity, h->stream));
+    s.blob_radius, h->bb, handle_split(h), h->stream));
   FR_CUDA(cudaMemsetAsync(h->work_counter, 0, sizeof(int), h->stream));
   FR_CUDA(cudaStreamWaitEvent(h->stream, h->band_join, 0));
   frb::InsertParams P{};

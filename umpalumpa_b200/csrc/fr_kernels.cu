@@ -438,13 +438,13 @@ __global__ void __launch_bounds__(256) batch_bin_kernel(const JobDesc *__restric
 }
 
 // Single-CTA planner: exclusive scan of the (brick, direction) counts into list offsets,
-// then cuts every brick's list into work items of at most `itemCap` entries, bricks taken
-// in `order` (heaviest expected first).  Sets status = FR_E_CAPACITY instead of
+// then cuts every brick's list into work items (ItemSplit), bricks taken in `order` (heaviest
+// expected first).  Sets status = FR_E_CAPACITY instead of
 // overflowing the list or item buffers.  When the status is already set (a space with a
 // projection outside the FFT payload, or an earlier failure), the fill pass writes no lists,
 // so no work items are published either: the insertion then reads no list entry.
 __global__ void __launch_bounds__(1024) plan_kernel(BinGeom g, const int *__restrict__ counts,
-  int *__restrict__ offsets, const int *__restrict__ order, int itemCap, int64_t listCap,
+  int *__restrict__ offsets, const int *__restrict__ order, ItemSplit split, int64_t listCap,
   int64_t itemsCap, WorkItem *__restrict__ items, int *__restrict__ nItems, int *__restrict__ status,
   unsigned long long *__restrict__ stats, const JobDesc *__restrict__ jobs, int nJobs)
 {
@@ -472,6 +472,21 @@ __global__ void __launch_bounds__(1024) plan_kernel(BinGeom g, const int *__rest
   }
   if (tid == 0) offsets[M] = int(min(total, (long long)listCap));
   __syncthreads();
+  // capacity of an item
+  int itemCap = split.cap;
+  if (split.want > 0) {  // uniform
+    __shared__ int longest;
+    if (tid == 0) longest = 0;
+    __syncthreads();
+    int len = 0;
+    if (split.perBrick > 0)
+      for (int b = tid; b < g.n_bricks; b += T) len = max(len, offsets[3 * b + 3] - offsets[3 * b]);
+    if (len > 0) atomicMax(&longest, len);
+    __syncthreads();
+    const long long shared = max((long long)split.least, (total + split.want - 1) / split.want);
+    const int whole = split.perBrick > 0 ? (longest + split.perBrick - 1) / split.perBrick : 0;
+    itemCap = int(min((long long)split.cap, max(shared, (long long)whole)));
+  }
   // pass 2: items per brick in `order`
   const int NB = g.n_bricks;
   const int perb = (NB + T - 1) / T;
@@ -570,7 +585,7 @@ cudaError_t launch_traverse_spaces(const float *rot, int64_t n, uint32_t imgX, u
 }
 
 cudaError_t launch_batch_binning(const JobDesc *jobs, int nJobs, int totalSpaces, int totalBricks,
-  int totalGroups, bool fast, float radius, const BinBuffers &b, int itemCap, cudaStream_t st)
+  int totalGroups, bool fast, float radius, const BinBuffers &b, const ItemSplit &split, cudaStream_t st)
 {
   const float hw = fast ? 2.5f : radius + 1e-3f;
   const float xmin = fast ? -1e-3f : -radius - 1e-3f;
@@ -582,7 +597,7 @@ cudaError_t launch_batch_binning(const JobDesc *jobs, int nJobs, int totalSpaces
   batch_bin_kernel<false><<<totalGroups, 256, 0, st>>>(jobs, nJobs, b.prep, b.counts, nullptr, nullptr, b.status);
   BinGeom g{};
   g.n_bricks = totalBricks;
-  plan_kernel<<<1, 1024, 0, st>>>(g, b.counts, b.offsets, b.order, itemCap, b.listCap, b.itemsCap, b.items,
+  plan_kernel<<<1, 1024, 0, st>>>(g, b.counts, b.offsets, b.order, split, b.listCap, b.itemsCap, b.items,
     b.nItems, b.status, b.stats, jobs, nJobs);
   batch_bin_kernel<true><<<totalGroups, 256, 0, st>>>(jobs, nJobs, b.prep, nullptr, b.offsets, b.list, b.status);
   return cudaGetLastError();
@@ -708,7 +723,7 @@ cudaError_t launch_batch_band(const JobDesc *jobs, int nJobs, int64_t totalUnits
 }
 
 cudaError_t launch_binning(const BinGeom &g, const fr_traverse_space *spaces, int n, int nProj,
-  bool fast, float radius, const BinBuffers &b, int itemCap, cudaStream_t st)
+  bool fast, float radius, const BinBuffers &b, const ItemSplit &split, cudaStream_t st)
 {
   const float hw = fast ? 2.5f : radius + 1e-3f;
   const float xmin = fast ? -1e-3f : -radius - 1e-3f;
@@ -719,10 +734,26 @@ cudaError_t launch_binning(const BinGeom &g, const fr_traverse_space *spaces, in
     b.prep, b.rec, b.status);
   const int blocks = (g.n_bricks + 7) / 8;
   bin_kernel<false><<<blocks, 256, 0, st>>>(g, b.prep, n, b.counts, nullptr, nullptr, b.status);
-  plan_kernel<<<1, 1024, 0, st>>>(g, b.counts, b.offsets, b.order, itemCap, b.listCap, b.itemsCap,
+  plan_kernel<<<1, 1024, 0, st>>>(g, b.counts, b.offsets, b.order, split, b.listCap, b.itemsCap,
     b.items, b.nItems, b.status, b.stats, nullptr, 0);
   bin_kernel<true><<<blocks, 256, 0, st>>>(g, b.prep, n, nullptr, b.offsets, b.list, b.status);
   return cudaGetLastError();
+}
+
+// Few spaces on few bricks left most brick groups idle: a group inserts one entry of its item
+// after the other (1.5-2.6 us each), so 64 spaces into 33^3 (27 bricks, 774 entries) took
+// 171 us on 27 groups.  Cutting the lists so that every group of the launch gets about four items
+// (at least two entries each: a flush costs about two) measured, whole calls, before -> after:
+// box 32 x 64 240 -> 67 us, box 64 x 2,000 in three calls 4.22 -> 0.70 ms, box 96 x 777 2.21 ->
+// 0.51 ms, box 256 x 1,537 in two calls 4.17 -> 3.70 ms.  Two, eight and sixteen items per group
+// ran 556, 507 and 534 us at box 96 and 3.70, 3.75 and 3.81 ms at box 256.  From about 900,000
+// entries (1,400 box-256 projections) on, the capacity of 512 is the shorter one.
+// Kahan accumulators: an item's sums reach the volume by plain adds, so a brick is cut into
+// eight items at most (besides those of the capacity), which keeps them at FP32's last bits.
+ItemSplit item_split(int itemCapacity, int brickGroups, const InsertConfig &cfg)
+{
+  const int perGroup = cfg.fast ? kFastItemsPerGroup : kItemsPerGroup;
+  return { itemCapacity, itemCapacity == kItemCapacity ? perGroup * brickGroups : 0, cfg.fast ? 32 : 2, cfg.kahan ? 8 : 0 };
 }
 
 int insert_max_groups(const InsertConfig &cfg) { return cfg.kahan ? 2 : 3; }

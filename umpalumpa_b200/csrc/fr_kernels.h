@@ -38,6 +38,24 @@ struct BinBuffers {
   int64_t itemsCap;
 };
 
+// How the plan cuts the binned lists into work items: at most `cap` list entries per item and,
+// where `want` > 0, so few that the launch's brick groups get about `want` items between them,
+// but at least `least` entries, and (`perBrick` > 0) no brick is cut into more than `perBrick`
+// items for it.
+struct ItemSplit {
+  int cap;
+  int want;
+  int least;
+  int perBrick;
+};
+
+// The default item capacity; only with it does the plan shorten items (`want` > 0), any other
+// capacity (fr_set_launch_params, the autotuner) is taken as given.
+constexpr int kItemCapacity = 512;
+constexpr int kItemsPerGroup = 4;
+constexpr int kFastItemsPerGroup = 1;  // nearest pixel: an entry costs a tenth of a blob entry
+
+
 struct InsertParams {
   const JobDesc *jobs;  // batched launches: the job table (the per-job fields below unused)
   void *volume;
@@ -79,6 +97,8 @@ struct InsertConfig {
   bool banded;  // half-planes in 4-row bands (always for a batch); else row-major
 };
 
+ItemSplit item_split(int itemCapacity, int brickGroups, const InsertConfig &cfg);
+
 using InsertFn = void (*)(InsertParams);
 // One insertion-kernel variant per storage type and layout, each in its own translation unit.
 InsertFn pick_insert_fp32(const InsertConfig &cfg);
@@ -119,12 +139,13 @@ cudaError_t launch_band_projections(const void *src, void *dst, int64_t n, int f
 // The same for every job of a batch: job j's projections go from its `src` to its `fft`, its
 // bands numbered from its `unitBase` (totalUnits bands in all).
 cudaError_t launch_batch_band(const JobDesc *jobs, int nJobs, int64_t totalUnits, int elemBytes, cudaStream_t st);
+// `split`: see ItemSplit.
 cudaError_t launch_binning(const BinGeom &g, const fr_traverse_space *spaces, int n, int nProj,
-  bool fast, float radius, const BinBuffers &b, int itemCap, cudaStream_t st);
+  bool fast, float radius, const BinBuffers &b, const ItemSplit &split, cudaStream_t st);
 // Binning of a batch: jobs (device job table, nJobs entries) with totalSpaces spaces,
 // totalBricks bricks and totalGroups 8-brick binning groups in all.
 cudaError_t launch_batch_binning(const JobDesc *jobs, int nJobs, int totalSpaces, int totalBricks,
-  int totalGroups, bool fast, float radius, const BinBuffers &b, int itemCap, cudaStream_t st);
+  int totalGroups, bool fast, float radius, const BinBuffers &b, const ItemSplit &split, cudaStream_t st);
 cudaError_t launch_insert(const InsertParams &P, const InsertConfig &cfg, int grid, cudaStream_t st);
 size_t insert_smem_bytes(const InsertConfig &cfg, int tableElems);
 int insert_groups(const InsertConfig &cfg);      // 256-thread groups per insertion CTA

@@ -32,7 +32,7 @@ namespace {
 
 constexpr size_t kScratchBytes = size_t(32) << 20;  // 32 MiB per device
 constexpr int kMaxDevices = 64;
-constexpr int kItemCapacity = 512;
+using frb::kItemCapacity;
 
 static __device__ __align__(256) unsigned char g_noalloc_scratch[kScratchBytes];
 
@@ -178,7 +178,7 @@ extern "C" int fr_insert_noalloc(int device, void *stream, const fr_dims *d, con
   chunk = std::min<int64_t>(chunk, int64_t(nSpaces));
   if (chunk < 1) return fail(FR_E_UNSUPPORTED, "volume too large for the 32 MiB scratch");
   const int64_t listCap = chunk * perSpace;
-  const int64_t itemsCap = listCap / kItemCapacity + g.n_bricks + 1;
+  int64_t itemsCap = listCap / kItemCapacity + g.n_bricks + 1;
   const size_t oPrep = off;
   off += align256(size_t(chunk) * frb::kSpacePrepBytes);
   const size_t oRec = off;
@@ -188,6 +188,9 @@ extern "C" int fr_insert_noalloc(int device, void *stream, const fr_dims *d, con
   const size_t oItems = off;
   off += align256(size_t(itemsCap) * frb::kWorkItemBytes);
   if (off > kScratchBytes) return fail(FR_E_UNSUPPORTED, "volume too large for the 32 MiB scratch");
+  // what is left of the array takes the items of a finer split (few spaces, idle brick groups)
+  const int64_t spareItems = int64_t((kScratchBytes - off) / frb::kWorkItemBytes);
+  itemsCap += spareItems;
 
   char *sb = static_cast<char *>(base);
   int *misc = reinterpret_cast<int *>(sb + oMisc);
@@ -228,6 +231,8 @@ extern "C" int fr_insert_noalloc(int device, void *stream, const fr_dims *d, con
     return fail(FR_E_CUDA, cudaGetErrorString(e));
   }
   if (occ < 1) return fail(FR_E_UNSUPPORTED, "insertion kernel does not fit on an SM");
+  frb::ItemSplit split = frb::item_split(kItemCapacity, sms * occ * frb::insert_groups(cfg), cfg);
+  split.want = int(std::min<int64_t>(split.want, spareItems));
 
   frb::InsertParams P{};
   P.volume = volume;
@@ -263,7 +268,7 @@ extern "C" int fr_insert_noalloc(int device, void *stream, const fr_dims *d, con
   P.cz = g.cz;
   for (uint64_t s0 = 0; s0 < nSpaces && e == cudaSuccess; s0 += uint64_t(chunk)) {
     const int n = int(std::min<uint64_t>(uint64_t(chunk), nSpaces - s0));
-    e = frb::launch_binning(g, spaces + s0, n, int(nProj), cfg.fast, s->blob_radius, bb, kItemCapacity, st);
+    e = frb::launch_binning(g, spaces + s0, n, int(nProj), cfg.fast, s->blob_radius, bb, split, st);
     if (e == cudaSuccess) e = cudaMemsetAsync(workCounter, 0, sizeof(int), st);
     if (e == cudaSuccess) e = frb::launch_insert(P, cfg, sms * occ, st);
   }

@@ -168,7 +168,7 @@ std::vector<Candidate> candidates(fr_handle *h, Candidate *def)
   const int maxg = frb::insert_max_groups(cfg);
   def->groups = maxg;
   def->ctas = 1;
-  def->item = 512;
+  def->item = frb::kItemCapacity;
   for (int g = 1; g <= maxg; ++g) {
     cfg.groups = g;
     const size_t smem = frb::insert_smem_bytes(cfg, tableElems);
