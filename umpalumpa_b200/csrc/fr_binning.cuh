@@ -25,10 +25,11 @@ __device__ __forceinline__ bool prep_space(const fr_traverse_space &s, float hal
   const int ua = dir == FR_DIR_YZ ? 1 : 0;
   const int va = dir == FR_DIR_XY ? 1 : 2;
   const int wa = dir == FR_DIR_XY ? 2 : (dir == FR_DIR_XZ ? 1 : 0);
-  r.lo0 = lo[ua];
-  r.hi0 = hi[ua];
-  r.lo1 = lo[va];
-  r.hi1 = hi[va];
+  const int far = 1 << 24;  // floats hold every integer up to here
+  r.lo0 = float(min(max(lo[ua], -far), far));
+  r.hi0 = float(min(max(hi[ua], -far), far));
+  r.lo1 = float(min(max(lo[va], -far), far));
+  r.hi1 = float(min(max(hi[va], -far), far));
   lo[wa] = -open;
   hi[wa] = open;
   for (int k = 0; k < 3; ++k) {
@@ -57,11 +58,20 @@ __device__ __forceinline__ bool prep_space(const fr_traverse_space &s, float hal
     r.wv = 0.f;
     r.hw = 1e9f;
   }
+  // half-space x' >= -r, with a margin of 0.01 in x' (far above the float error of h at the
+  // largest volume, 1.5e-3 in x')
   const double t0[3] = { s.transformInv[0][0], s.transformInv[0][1], s.transformInv[0][2] };
-  r.xu = float(t0[ua]);
-  r.xv = float(t0[va]);
-  r.xw = float(t0[wa]);
-  r.xwInv = fabs(t0[wa]) > 1e-3 ? float(1.0 / t0[wa]) : 0.f;
+  const double tw = t0[wa];
+  r.h0 = -1e30f;
+  r.hu = 0.f;
+  r.hv = 0.f;
+  if (fabs(tw) > 1e-3) {
+    r.h0 = float(c[wa] + (t0[ua] * c[ua] + t0[va] * c[va] - double(radius) - 0.01) / tw);
+    r.hu = float(-t0[ua] / tw);
+    r.hv = float(-t0[va] / tw);
+    if (tw < 0) r.hw = -r.hw;
+  }
+  r.sphere = s.maxDistanceSqr;
   const float *un = s.unitNormal, *bo = s.bottomOrigin;
   r.nu = un[ua];
   r.nv = un[va];
@@ -69,8 +79,7 @@ __device__ __forceinline__ bool prep_space(const fr_traverse_space &s, float hal
   r.bu = bo[ua];
   r.bv = bo[va];
   r.bw = bo[wa];
-  r.dir = bad ? -1 : dir;
-  r.pad = 0;
+  r.pad[0] = r.pad[1] = 0;
   return !bad;
 }
 

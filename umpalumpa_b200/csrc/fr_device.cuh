@@ -44,29 +44,29 @@ static_assert(sizeof(SpacePrep) == 64, "SpacePrep is 64 bytes");
 // Per-space record read by the insertion kernel (128 bytes = eight 16-byte loads), built
 // once per space by the binning prep pass.  The axes U, V are the traversal plane of the
 // space's direction and W its column axis (XY: x, y | z;  XZ: x, z | y;  YZ: y, z | x).
-//  - T, maxDist2, weight, proj: as in the TraverseSpace.
-//  - lo0/hi0/lo1/hi1: the traversal AABB on U and V (fr_cpu_kernels.hpp:166-238).
+//  - T, maxDist2, weight, proj: as in the TraverseSpace (the voxels' part, three loads).
+//  - lo0/hi0/lo1/hi1: the traversal AABB on U and V (fr_cpu_kernels.hpp:166-238), as floats
+//    (clamped to 2^24, beyond every volume).
 //  - w0, wu, wv, hw (blob mode): the slab |t2.(q - c)| <= r crosses column (U, V) at
-//    W = w0 + wu U + wv V with half-width hw along W (plus a margin).  A voxel contributes
+//    W = w0 + wu U + wv V with half-width |hw| along W (plus a margin).  A voxel contributes
 //    only if its float |t2.(q - c)| <= r, and the reference's column range
 //    [floor(min(z1,z2)), ceil(max(z1,z2))] always contains every such voxel, so visiting
 //    [ceil(wc - hw), floor(wc + hw)] instead yields the same contributing voxels.
+//  - h0, hu, hv (blob mode): a voxel contributes only if its image x' = t0.(q - c) >= -r, which
+//    bounds column (U, V) at W = h0 + hu U + hv V: from below where hw is positive, from
+//    above where it is negative; h0 = -1e30 where t0 has no component along W.  sphere = maxDist2.
 //  - nu, nv, nw, bu, bv, bw (nearest mode): the plane normal and bottom origin on U, V, W,
 //    for the reference's exact rounded plane hit.
-//  - xu, xv, xw, xwInv: row 0 of transformInv on U, V, W; a voxel contributes only if its
-//    image x' = t0.(q - c) >= -r (>= 0 in nearest mode), which bounds each column on one side.
 struct SpaceRec {
   float T[9];
   float maxDist2;
   float weight;
   int proj;
-  int lo0, hi0, lo1, hi1;
+  float lo0, hi0, lo1, hi1;
   float w0, wu, wv, hw;
+  float h0, hu, hv, sphere;
   float nu, nv, nw, bu, bv, bw;
-  float xu, xv;         // half-space x' >= -r per column: row 0 of transformInv on U, V,
-  float xwInv, xw;      // 1/t0_W (0 when |t0_W| <= 1e-3) and t0_W
-  int dir;
-  int pad;
+  int pad[2];
 };
 static_assert(sizeof(SpaceRec) == 128, "SpaceRec is 128 bytes");
 

@@ -17,11 +17,20 @@
 // Work split: a CTA runs several independent 256-thread groups, each working on its own
 // brick (Groups below); a batched launch (JOBS) takes the items of several jobs, each item
 // naming its job in the job table.  Warp w of a group owns the 32 brick columns (U, V) = (tx, w + 8 ty),
-// tx < 16, ty < 2, of the current direction.  Per projection each lane finds its column's voxel range;
-// the warp then deals the warp's voxels out to its lanes 32 at a time (prefix sum + binary
-// search over shuffles), so lanes stay busy whatever the column lengths.  Within one
+// tx < 16, ty < 2, of the current direction.  Per projection each lane finds its column's voxel
+// range; the warp deals the voxels of its projections, one projection after the other, to its
+// lanes and runs them 32 at a time (insert_blobs), so that a step is full whatever the column
+// lengths and wherever one projection's voxels end.  Within one
 // direction a warp touches only its own columns, so projections need no synchronisation
 // beyond __syncwarp; a group synchronises (named barrier) only when the direction changes.
+//
+// What bounds it (lookup, FP32, banded, 1,537-20,000 projections at box 256): the L1/shared data
+// path (117 wavefronts per step of 32 voxels: 60 pixel gathers, 34 table lookups, 13 accumulators)
+// at 73 % and instruction issue at 66 %, with the 24 warps that shared memory and registers
+// allow.  Against steps that start anew for every projection (26 of 32 lanes filled, the source
+// columns found by a binary search over shuffles), with one voxel body per direction instead of
+// one for all: 19 % fewer instructions and 13 % fewer wavefronts; 20,000 projections
+// 45.8 -> 37.5 ms.
 //
 // Half-plane layouts (BANDED): the caller's row-major half-planes, or the same pixels in bands
 // of four rows stored column by column (pixel (y, x) at (y / 4) * bandStride + 4 x + y % 4,
@@ -37,22 +46,15 @@ namespace frb {
 
 enum { kModeLut = 0, kModeFastKaiser = 1, kModeKaiser = 2, kModeKaiserTable = 3 };
 
-// Traversal plane axes (U, V) and column axis W per direction (traverse_space.hpp:24-28).
-template<int DIR> struct Axes;
-template<> struct Axes<FR_DIR_XY> { static constexpr int U = 0, V = 1, W = 2; };
-template<> struct Axes<FR_DIR_XZ> { static constexpr int U = 0, V = 2, W = 1; };
-template<> struct Axes<FR_DIR_YZ> { static constexpr int U = 1, V = 2, W = 0; };
-
-template<int K, typename T> __device__ __forceinline__ T pick3(T a, T b, T c)
+// A brick's voxel (x, y, z) has the linear index 256 z + 16 y + x; its accumulators sit at that
+// index with the low five bits -- the shared-memory bank -- rotated by 5 (y / 2) + 6 z, so that
+// the voxels of a step (short runs along x, y or z in two rows of columns) spread over all 32
+// banks: 2.1 wavefronts per access of a full step, where swizzling x by z + y / 2 alone, which
+// keeps the rows y and y + 8 of a warp in the same 16 banks, took 3.6 (simulated over the dealing
+// at box 256; the rotations with 5..9 in place of 5 and 6 are within 4 %).
+__device__ __forceinline__ int acc_slot(int lin)
 {
-  return K == 0 ? a : (K == 1 ? b : c);
-}
-
-// Brick accumulators are [z][y][x] with x swizzled by (z + y/2) mod 16, so that the voxels
-// of any x-, y- or z-column fall into distinct shared-memory banks.
-__device__ __forceinline__ int acc_index(int x, int y, int z)
-{
-  return (z * kBrick + y) * kBrick + (x ^ ((z + (y >> 1)) & (kBrick - 1)));
+  return (lin & ~31) | ((lin + 5 * ((lin >> 5) & 7) + 6 * (lin >> 8)) & 31);
 }
 
 // Sizes and payloads of the job a work item belongs to.  A single-job launch builds it from
@@ -113,109 +115,129 @@ __device__ __forceinline__ JobGeom geom_of(const JobDesc &J)
 }
 
 struct Accum {
-  float *re, *im, *w;              // brick accumulators
-  __nv_bfloat16 *cre, *cim, *cw;   // Kahan compensations (KAHAN only)
+  float2 *v;              // brick accumulators: the complex values
+  float *w;               // and the weights
+  __nv_bfloat162 *cv;     // Kahan compensations (KAHAN only)
+  __nv_bfloat16 *cw;
 };
 
-// Kahan-compensated add.  The compensation -- the rounding error of the previous add, at most
-// half an ulp of the sum -- is kept in BF16: its 8 significant bits leave each add at most
-// 1/256 of plain FP32's rounding residual, and 18 instead of 24 bytes per voxel let the blob
-// table stay in shared memory beside two brick groups.
-template<bool KAHAN>
-__device__ __forceinline__ void acc_add(float *sum, __nv_bfloat16 *comp, int i, float v)
+// Kahan-compensated add; returns the new sum.  The compensation -- the rounding error of the
+// previous add, at most half an ulp of the sum -- is kept in BF16: its 8 significant bits leave
+// each add at most 1/256 of plain FP32's rounding residual, and 18 instead of 24 bytes per voxel
+// let the blob table stay in shared memory beside two brick groups.
+__device__ __forceinline__ float kahan_add(float sum, float &comp, float v)
 {
-  if (KAHAN) {
-    const float y = __fsub_rn(v, __bfloat162float(comp[i]));
-    const float t = __fadd_rn(sum[i], y);
-    comp[i] = __float2bfloat16_rn(__fsub_rn(__fsub_rn(t, sum[i]), y));
-    sum[i] = t;
-  } else {
-    sum[i] += v;
-  }
+  const float y = __fsub_rn(v, comp);
+  const float t = __fadd_rn(sum, y);
+  comp = __fsub_rn(__fsub_rn(t, sum), y);
+  return t;
 }
 
-// The fields of a SpaceRec the kernel reads, loaded with 16-byte broadcast loads: load_rec
-// reads what the column phase needs, run_direction the voxel fields after it (the rotation, in
-// banded kernels, for every voxel: load_rotation).
-struct RecView {
+template<bool KAHAN>
+__device__ __forceinline__ void acc_add(const Accum &A, int i, float2 v, float w)
+{
+  float2 s = A.v[i];
+  if (KAHAN) {
+    float2 c = __bfloat1622float2(A.cv[i]);
+    float cw = __bfloat162float(A.cw[i]);
+    s.x = kahan_add(s.x, c.x, v.x);
+    s.y = kahan_add(s.y, c.y, v.y);
+    A.w[i] = kahan_add(A.w[i], cw, w);
+    A.cv[i] = __floats2bfloat162_rn(c.x, c.y);
+    A.cw[i] = __float2bfloat16_rn(cw);
+  } else {
+    s.x += v.x;
+    s.y += v.y;
+    A.w[i] += w;
+  }
+  A.v[i] = s;
+}
+
+// Voxels a warp's list holds (insert_blobs): an entry has at most 32 columns x 16, nearly always
+// fewer than 120.  24 lists of 240 16-bit voxels leave three plain brick groups and a
+// 10,000-entry table in the 196 KB shared-memory carve-out, so the L1 keeps its size.
+constexpr int kVoxelList = 240;
+
+__device__ __forceinline__ float approx_sqrt(float v)
+{
+  float r;
+  asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(v));
+  return r;
+}
+
+// The fields of a SpaceRec a voxel needs (every voxel of a step may belong to another space).
+struct VoxelRec {
   float T[9];
   float maxDist2, weight;
   int proj;
-  int lo0, hi0, lo1, hi1;
-  float w0, wu, wv, hw;
-  float nu, nv, nw, bu, bv, bw;
-  float xu, xv, xw, xwInv;
 };
 
-template<bool FAST>
-__device__ __forceinline__ void load_rec(const SpaceRec *r, RecView &v)
+__device__ __forceinline__ VoxelRec load_voxel_rec(const SpaceRec *r)
 {
   const float4 *q = reinterpret_cast<const float4 *>(r);
-  const float4 f2 = __ldg(q + 2), f3 = __ldg(q + 3);
-  const float4 f4 = __ldg(q + 4);
-  v.maxDist2 = f2.y;
-  v.lo0 = __float_as_int(f3.x);
-  v.hi0 = __float_as_int(f3.y);
-  v.lo1 = __float_as_int(f3.z);
-  v.hi1 = __float_as_int(f3.w);
-  v.w0 = f4.x; v.wu = f4.y; v.wv = f4.z; v.hw = f4.w;
-  if (FAST) {
-    const float4 f5 = __ldg(q + 5), f6 = __ldg(q + 6);
-    v.nu = f5.x; v.nv = f5.y; v.nw = f5.z; v.bu = f5.w; v.bv = f6.x; v.bw = f6.y;
-  } else {
-    const float4 f6 = __ldg(q + 6), f7 = __ldg(q + 7);
-    v.xu = f6.z; v.xv = f6.w; v.xwInv = f7.x; v.xw = f7.y;
-  }
+  const float4 f0 = __ldg(q), f1 = __ldg(q + 1), f2 = __ldg(q + 2);
+  return { { f0.x, f0.y, f0.z, f0.w, f1.x, f1.y, f1.z, f1.w, f2.x }, f2.y, f2.z, __float_as_int(f2.w) };
 }
 
-// The nine entries of transformInv (the record's first 36 bytes).  Volatile, so that the
-// compiler re-reads them where they are used instead of keeping them live in registers.
-__device__ __forceinline__ void load_rotation(const float4 *rec, float *T)
-{
-  asm volatile("ld.global.nc.v4.f32 {%0, %1, %2, %3}, [%4];"
-               : "=f"(T[0]), "=f"(T[1]), "=f"(T[2]), "=f"(T[3]) : "l"(rec));
-  asm volatile("ld.global.nc.v4.f32 {%0, %1, %2, %3}, [%4];"
-               : "=f"(T[4]), "=f"(T[5]), "=f"(T[6]), "=f"(T[7]) : "l"(rec + 1));
-  asm volatile("ld.global.nc.f32 %0, [%1];" : "=f"(T[8]) : "l"(rec + 2));
-}
+// Coordinate of voxel i (0..15) of the brick relative to the volume centre, as a float: exact.
+// `origin` is the brick's first coordinate relative to the centre less 2^23 (brick_origin), so
+// that the integer is placed in the mantissa and one subtraction converts it.
+__device__ __forceinline__ float brick_origin(int o, int c) { return float(o - c) - 8388608.f; }
+__device__ __forceinline__ float voxel_coord(int i, float origin) { return __int_as_float(0x4b000000 | i) + origin; }
 
 // FR<>::ProcessVoxelBlob (fr_cpu_kernels.hpp:70-152) for voxel (X, Y, Z): Kaiser-Bessel
 // gather of the projection pixels within the blob radius.  The blob weights are summed raw
 // and scaled by the space weight (and the storage scale) once at the end.  Returns false if
 // the voxel is rejected.
 template<int MODE, int TAPS, int STORAGE, bool GENERIC, bool BANDED>
-__device__ __forceinline__ bool voxel_blob(const InsertParams &P, const JobGeom &G, const RecView &s,
-  const typename Pixel<STORAGE>::T *__restrict__ img, int bandStride, float scale, const float *lut, int X,
-  int Y, int Z, float &ore, float &oim, float &ow)
+__device__ __forceinline__ bool voxel_blob(const InsertParams &P, const JobGeom &G, const VoxelRec &s,
+  const typename Pixel<STORAGE>::T *__restrict__ img, int bandStride, float scale, const float *lut, float px,
+  float py, float pz, float2 &ov, float &ow)
 {
   const fr_constants &c = P.c;
-  const float px = float(X - G.cx), py = float(Y - G.cy), pz = float(Z - G.cz);
-  if (px * px + py * py + pz * pz > s.maxDist2) return false;  // integer-valued: exact
   const float qx = add_(add_(mul_(s.T[0], px), mul_(s.T[1], py)), mul_(s.T[2], pz));
   const float qy0 = add_(add_(mul_(s.T[3], px), mul_(s.T[4], py)), mul_(s.T[5], pz));
   const float qz = add_(add_(mul_(s.T[6], px), mul_(s.T[7], py)), mul_(s.T[8], pz));
   const float r = c.cBlobRadius;
-  if (qx < -r) return false;
   const float qy = add_(qy0, float(G.cy));
   const float rSq = mul_(r, r);
   const float zSq = mul_(qz, qz);
-  if (zSq > rSq) return false;
-  // no pixel lies within the blob radius (also rejects non-finite coordinates)
-  if (!(qx <= float(G.fftX) + r && qy >= -r && qy <= float(G.fftY) + r)) return false;
+  // The reference's rejection tests -- outside the frequency sphere (integer-valued: exact),
+  // behind the image, off the slab -- and those no pixel lies within the blob radius of (also
+  // rejects non-finite coordinates), as one predicate.
+  const bool inside = !(px * px + py * py + pz * pz > s.maxDist2) & !(qx < -r) & !(zSq > rSq)
+                      & (qx <= float(G.fftX) + r) & (qy >= -r) & (qy <= float(G.fftY) + r);
+  if (!inside) return false;
   // The TAPS x TAPS window starts at (ceil(qx - r), ceil(qy - r)) shifted into the image, so
   // it covers the reference's clamped blob box [max(ceil(q - r), 0), min(floor(q + r), X-1)]
   // and lies inside the image; candidates outside the blob box have d2 > r^2, so d2 <= r^2
   // is the only per-tap test (FR::ProcessVoxelBlob's radius test, fr_cpu_kernels.hpp:128-134).
   // GENERIC (a half-plane narrower or shorter than the window) tests the blob box explicitly.
-  int minX = max(int(ceilf(sub_(qx, r))), 0);
-  int minY = max(int(ceilf(sub_(qy, r))), 0);
-  const int maxX = min(int(floorf(add_(qx, r))), G.fftX - 1);
-  const int maxY = min(int(floorf(add_(qy, r))), G.fftY - 1);
+  // The origin stays a float (integer-valued, exact) for the distances and is converted once
+  // for the addresses.
+  float x0 = fmaxf(ceilf(sub_(qx, r)), 0.f);
+  float y0 = fmaxf(ceilf(sub_(qy, r)), 0.f);
   if (!GENERIC) {
-    minX = min(minX, G.fftX - TAPS);
-    minY = min(minY, G.fftY - TAPS);
+    x0 = fminf(x0, float(G.fftX - TAPS));
+    y0 = fminf(y0, float(G.fftY - TAPS));
   }
-  const float dx0 = sub_(qx, float(minX));
+  const int minX = int(x0), minY = int(y0);
+  const int maxX = min(int(floorf(add_(qx, r))), G.fftX - 1);  // GENERIC only
+  const int maxY = min(int(floorf(add_(qy, r))), G.fftY - 1);
+  const float dx0 = sub_(qx, x0);
+  // First pixel of window row ii.  Banded: rows o = minY % 4, o + 1, ... of the window's first
+  // band; row ii lies (o + ii) / 4 bands further (at most one for 4 rows), where the same row
+  // offset less 4 applies.
+  using PT = typename Pixel<STORAGE>::T;
+  const int o = BANDED ? minY & 3 : 0;
+  const PT *w0 = BANDED ? img + size_t(unsigned(minY) >> 2) * unsigned(bandStride) + unsigned(o + 4 * minX)
+                        : img + size_t(unsigned(minY)) * unsigned(G.fftX) + unsigned(minX);
+  const PT *w1 = w0 + (bandStride - 4);
+  auto window_row = [&](int ii) -> const PT * {
+    if (!BANDED) return w0 + size_t(ii) * unsigned(G.fftX);
+    if (TAPS == 4) return (o + ii >= 4 ? w1 : w0) + ii;
+    return w0 + size_t(unsigned(o + ii) >> 2) * unsigned(bandStride - 4) + ii;
+  };
   // Taps are evaluated in pairs with packed FP32x2 arithmetic: per pair one fused d2 and one
   // fused table position, per tap one fused complex accumulation.  Each lane rounds exactly
   // like the scalar fmaf it replaces.
@@ -228,7 +250,7 @@ __device__ __forceinline__ bool voxel_blob(const InsertParams &P, const JobGeom 
   const float2 half2 = make_float2(0.5f, 0.5f);
   float2 acc = make_float2(0.f, 0.f);
   float w = 0.f;
-  auto tap = [&](const typename Pixel<STORAGE>::T *row, int ii, int jj, float d2, float pos) {
+  auto tap = [&](const PT *row, int ii, int jj, float d2, float pos) {
     const bool inBox = !GENERIC || (minY + ii <= maxY && minX + jj <= maxX);
     if (inBox && d2 <= rSq) {
       float wb;
@@ -256,12 +278,10 @@ __device__ __forceinline__ bool voxel_blob(const InsertParams &P, const JobGeom 
   };
 #pragma unroll
   for (int ii = 0; ii < TAPS; ++ii) {
-    const float dy = sub_(qy, float(minY + ii));
+    const float dy = sub_(qy, add_(y0, float(ii)));
     const float yz = add_(mul_(dy, dy), zSq);
     const float2 yz2 = make_float2(yz, yz);
-    const int ry = minY + ii;
-    const typename Pixel<STORAGE>::T *row =
-      BANDED ? img + size_t(ry / 4) * size_t(bandStride) + (ry % 4) + 4 * minX : img + size_t(ry) * G.fftX + minX;
+    const PT *row = window_row(ii);
 #pragma unroll
     for (int k = 0; k < TAPS / 2; ++k) {
       const float2 d2 = __ffma2_rn(dxp[k], dxp[k], yz2);
@@ -275,20 +295,17 @@ __device__ __forceinline__ bool voxel_blob(const InsertParams &P, const JobGeom 
     }
   }
   const float dw = mul_(s.weight, scale);
-  const float2 o = __fmul2_rn(acc, make_float2(dw, dw));
-  ore = o.x;
-  oim = o.y;
+  ov = __fmul2_rn(acc, make_float2(dw, dw));
   ow = mul_(w, s.weight);
   return true;
 }
 
 // FR<>::ProcessVoxel (fr_cpu_kernels.hpp:18-68): nearest pixel.
 template<int STORAGE, bool BANDED>
-__device__ __forceinline__ bool voxel_nearest(const JobGeom &G, const RecView &s,
-  const typename Pixel<STORAGE>::T *__restrict__ img, int bandStride, float scale, int X, int Y, int Z,
-  float &ore, float &oim, float &ow)
+__device__ __forceinline__ bool voxel_nearest(const JobGeom &G, const VoxelRec &s,
+  const typename Pixel<STORAGE>::T *__restrict__ img, int bandStride, float scale, float px, float py, float pz,
+  float2 &ov, float &ow)
 {
-  const float px = float(X - G.cx), py = float(Y - G.cy), pz = float(Z - G.cz);
   if (px * px + py * py + pz * pz > s.maxDist2) return false;
   const float qx = add_(add_(mul_(s.T[0], px), mul_(s.T[1], py)), mul_(s.T[2], pz));
   const float qy = add_(add_(mul_(s.T[3], px), mul_(s.T[4], py)), mul_(s.T[5], pz));
@@ -299,128 +316,198 @@ __device__ __forceinline__ bool voxel_nearest(const JobGeom &G, const RecView &s
                                                : img + size_t(imgY) * G.fftX + imgX);
   const float w = s.weight;
   const float wt = mul_(w, scale);
-  ore = mul_(v.x, wt);
-  oim = mul_(v.y, wt);
+  ov = make_float2(mul_(v.x, wt), mul_(v.y, wt));
   ow = w;
   return true;
 }
 
-// All list entries [e0, e1) of one direction for the brick at (ox, oy, oz).
-template<int DIR, int MODE, int TAPS, bool FAST, int STORAGE, bool KAHAN, bool JOBS, bool BANDED>
-__device__ __forceinline__ void run_direction(const InsertParams &P, const JobGeom &G, const Accum &A,
-  const float *lut, int ox, int oy, int oz, int warp, int lane, int e0, int e1)
+// The brick at (ox, oy, oz) seen along one traversal direction (uniform across the group): the
+// plane axes U, V and the column axis W (traverse_space.hpp:24-28; XY: x, y | z;  XZ: x, z | y;
+// YZ: y, z | x), and this lane's column.
+struct Column {
+  float U, V;         // the column's volume coordinates
+  int lin, sW;        // linear brick index of its voxel at W = 0 (before the brick), step along W
+  bool in;            // inside the volume
+  int oW, wHi;        // first coordinate of the brick along W, last one inside the volume
+  float du, dv, cw;   // U, V relative to the centre; the centre along W
+};
+
+__device__ __forceinline__ Column column_of(const JobGeom &G, int dir, int ox, int oy, int oz, int warp, int lane)
 {
-  using AX = Axes<DIR>;
-  using PT = typename Pixel<STORAGE>::T;
-  const PT *fft = reinterpret_cast<const PT *>(G.fft);
-  // a single-job launch reads the band stride as a constant operand of the launch parameters
-  const int bandStride = JOBS ? G.bandStride : P.bandStride;
-  const size_t plane = BANDED ? size_t((G.fftY + 3) / 4) * size_t(bandStride) : size_t(G.fftX) * size_t(G.fftY);
-  const int oU = pick3<AX::U>(ox, oy, oz), oV = pick3<AX::V>(ox, oy, oz), oW = pick3<AX::W>(ox, oy, oz);
-  const int nU = pick3<AX::U>(G.vx, G.vy, G.vz), nV = pick3<AX::V>(G.vx, G.vy, G.vz);
-  const int nW = pick3<AX::W>(G.vx, G.vy, G.vz);
+  const bool xy = dir == FR_DIR_XY, yz = dir == FR_DIR_YZ;
   // warp w owns column rows w and w + 8: a slab that crosses part of the brick face spreads
   // over the warps instead of piling onto a few (2 % faster than adjacent rows)
   const int tu = lane & (kBrick - 1), tv = warp + 8 * (lane >> 4);
-  const int U = oU + tu, V = oV + tv;
-  const bool colIn = U < nU && V < nV;
-  const int wLo = oW, wHi = min(oW + kBrick, nW) - 1;
-  const float uf = float(U), vf = float(V);
-  const float du = float(U - pick3<AX::U>(G.cx, G.cy, G.cz)), dv = float(V - pick3<AX::V>(G.cx, G.cy, G.cz));
-  const float cw = float(pick3<AX::W>(G.cx, G.cy, G.cz));
-  const float r = P.c.cBlobRadius;
-  for (int e = e0; e < e1; ++e) {
-    const int si = __ldg(P.list + e);
-    RecView s;
-    load_rec<FAST>(P.recs + si, s);
-    // this lane's column range
-    int lo = 1, hi = 0;
-    if (colIn && U >= s.lo0 && U <= s.hi0 && V >= s.lo1 && V <= s.hi1) {
-      if (FAST) {
-        lo = hi = int(add_(plane_hit(uf, vf, s.nu, s.nv, s.nw, s.bu, s.bv, s.bw), 0.5f));
-      } else {
-        // slab |t2.p| <= r, frequency sphere |p|^2 <= maxDist2 and image half-space
-        // t0.p >= -r, each widened by a margin; the voxel checks decide exactly
-        const float wc = fmaf(s.wu, uf, fmaf(s.wv, vf, s.w0));
-        float flo = wc - s.hw, fhi = wc + s.hw;
-        const float rem = s.maxDist2 - du * du - dv * dv;
-        const float sq = sqrtf(fmaxf(rem, 0.f)) + 1e-3f;
-        flo = fmaxf(flo, cw - sq);
-        fhi = fminf(fhi, cw + sq);
-        if (s.xwInv != 0.f) {
-          const float b = cw + (-r - 0.01f - s.xu * du - s.xv * dv) * s.xwInv;
-          if (s.xw > 0.f) flo = fmaxf(flo, b);
-          else fhi = fminf(fhi, b);
+  const int U = (yz ? oy : ox) + tu, V = (xy ? oy : oz) + tv;
+  Column c;
+  c.U = float(U);
+  c.V = float(V);
+  c.in = U < (yz ? G.vy : G.vx) && V < (xy ? G.vy : G.vz);
+  c.oW = xy ? oz : (yz ? ox : oy);
+  c.wHi = min(c.oW + kBrick, xy ? G.vz : (yz ? G.vx : G.vy)) - 1;
+  c.sW = xy ? 256 : (yz ? 1 : 16);
+  c.lin = tu * (yz ? 16 : 1) + tv * (xy ? 16 : 256) - c.oW * c.sW;
+  c.du = float(U - (yz ? G.cy : G.cx));
+  c.dv = float(V - (xy ? G.cy : G.cz));
+  c.cw = float(xy ? G.cz : (yz ? G.cx : G.cy));
+  return c;
+}
+
+// All list entries [e0, e1) of one direction for the brick at (ox, oy, oz), blob insertion.
+//
+// The voxels of the entries form one stream per warp, in entry order: every lane lists its
+// column's voxels of an entry in the warp's shared-memory list (at the prefix sum of the column
+// lengths), the lanes from `n` on take them from there, and a step runs when all 32 lanes hold
+// one (or the entries have ended).  A step that starts anew for every entry fills 26 of 32 lanes
+// at box 256 (24 at box 64); the stream fills all of them, with 1.4 entries per step.  Two entries of a
+// step may hold the same voxel, so their adds follow one another (`part` numbers the entries of
+// the step).
+template<int MODE, int TAPS, int STORAGE, bool KAHAN, bool JOBS, bool BANDED>
+__device__ __forceinline__ void insert_blobs(const InsertParams &P, const JobGeom &G, const Accum &A,
+  const float *lut, uint16_t *list, int ox, int oy, int oz, int dir, int warp, int lane, int e0, int e1)
+{
+  using PT = typename Pixel<STORAGE>::T;
+  // a single-job launch reads the band stride as a constant operand of the launch parameters
+  const int bandStride = JOBS ? G.bandStride : P.bandStride;
+  const size_t plane = BANDED ? size_t((G.fftY + 3) / 4) * size_t(bandStride) : size_t(G.fftX) * size_t(G.fftY);
+  const Column col = column_of(G, dir, ox, oy, oz, warp, lane);
+  const float bx = brick_origin(ox, G.cx), by = brick_origin(oy, G.cy), bz = brick_origin(oz, G.cz);
+  // the column inside the brick and the frequency sphere |p|^2 <= sphere (with a margin), kept
+  // while the entries' spheres are alike -- as they are in a reconstruction
+  float sphere = nanf(""), clipLo = 0.f, clipHi = 0.f;
+  int n = 0, parts = 0;        // lanes that hold a voxel, entries they come from
+  int voxel = 0, space = 0;    // this lane's: linear brick index | part << 12, space
+  int at = 0, have = 0;        // the list: voxels taken, voxels listed
+  int si = 0;                  // the space they belong to
+  int listed = 0;              // voxels of entry e listed before (an entry longer than the list)
+  for (int e = e0;;) {
+    while (n < 32) {
+      if (at == have) {  // list the next entry: this lane's column range
+        if (e == e1) break;
+        si = __ldg(P.list + e);
+        const float4 *q = reinterpret_cast<const float4 *>(P.recs + si);
+        const float4 box = __ldg(q + 3), slab = __ldg(q + 4), half = __ldg(q + 5);
+        if (half.w != sphere) {  // uniform
+          sphere = half.w;
+          const float rem = sphere - col.du * col.du - col.dv * col.dv;
+          const float sq = approx_sqrt(fmaxf(rem, 0.f)) + 8e-3f;
+          const bool hit = col.in && rem >= 0.f;
+          clipLo = hit ? fmaxf(col.cw - sq, float(col.oW)) : 1e9f;
+          clipHi = hit ? fminf(col.cw + sq, float(col.wHi)) : -1e9f;
         }
-        lo = rem >= 0.f ? int(ceilf(flo)) : 1;
-        hi = rem >= 0.f ? int(floorf(fhi)) : 0;
-      }
-      lo = max(lo, wLo);
-      hi = min(hi, wHi);
-    }
-    const int cnt = max(hi - lo + 1, 0);
-    // warp prefix sum of the column lengths
-    int incl = cnt;
+        // slab |t2.p| <= r and image half-space t0.p >= -r, with margins; the voxel checks
+        // decide exactly
+        const float wc = fmaf(slab.y, col.U, fmaf(slab.z, col.V, slab.x));
+        const float hb = fmaf(half.y, col.U, fmaf(half.z, col.V, half.x));
+        float flo = fmaxf(wc - fabsf(slab.w), clipLo), fhi = fminf(wc + fabsf(slab.w), clipHi);
+        if (slab.w > 0.f) flo = fmaxf(flo, hb);
+        else fhi = fminf(fhi, hb);
+        const int lo = int(ceilf(flo)), hi = int(floorf(fhi));
+        const bool hit = col.U >= box.x && col.U <= box.y && col.V >= box.z && col.V <= box.w && lo <= hi;
+        // prefix sum of the column lengths (0..16) by bit planes; a blob of radius < 2 gives at
+        // most 7 voxels per column where the normal's component along W dominates
+        const int cnt = hit ? hi - lo + 1 : 0;
+        const unsigned before = (1u << lane) - 1u;
+        const unsigned b0 = __ballot_sync(0xffffffffu, cnt & 1), b1 = __ballot_sync(0xffffffffu, cnt & 2),
+                       b2 = __ballot_sync(0xffffffffu, cnt & 4), b3 = __ballot_sync(0xffffffffu, cnt & 24);
+        int excl = __popc(b0 & before) + 2 * __popc(b1 & before) + 4 * __popc(b2 & before);
+        int total = __popc(b0) + 2 * __popc(b1) + 4 * __popc(b2);
+        int v = col.lin + lo * col.sW;
+        if (b3 == 0 && total <= kVoxelList) {
+          __syncwarp();  // the list's last voxels have been taken
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const int t = __shfl_up_sync(0xffffffffu, incl, o);
-      if (lane >= o) incl += t;
-    }
-    const int total = __shfl_sync(0xffffffffu, incl, 31);
-    if (total == 0) continue;  // warp-uniform
-    const int excl = incl - cnt;
-    // Banded kernels read the rotation rows again (L1 hits) for every voxel instead of holding
-    // them in registers through the voxel loop: they run at their register cap, and the nine
-    // registers let the tap loads of a voxel stay in flight together (6 % faster).  The
-    // row-major kernels keep them (re-reading costs them 3 %).
-    const float4 *rec4 = reinterpret_cast<const float4 *>(P.recs + si);
-    {
-      const float4 f2 = __ldg(rec4 + 2);
-      s.weight = f2.z;
-      s.proj = __float_as_int(f2.w);
-      if (!BANDED) {
-        const float4 f0 = __ldg(rec4), f1 = __ldg(rec4 + 1);
-        s.T[0] = f0.x; s.T[1] = f0.y; s.T[2] = f0.z; s.T[3] = f0.w;
-        s.T[4] = f1.x; s.T[5] = f1.y; s.T[6] = f1.z; s.T[7] = f1.w;
-        s.T[8] = f2.x;
-      }
-    }
-    const float scale = STORAGE == FR_STORAGE_FP32 ? 1.f : __ldg(G.scales + s.proj);
-    const PT *img = fft + size_t(s.proj) * plane;
-    for (int base = 0; base < total; base += 32) {
-      const int k = base + lane;
-      // source lane: the largest s with excl_s <= k
-      int src = 0;
-#pragma unroll
-      for (int step = 16; step >= 1; step >>= 1) {
-        const int ex = __shfl_sync(0xffffffffu, excl, src + step);
-        if (ex <= k) src += step;
-      }
-      const int wv = __shfl_sync(0xffffffffu, lo, src) + (k - __shfl_sync(0xffffffffu, excl, src));
-      if (k < total) {
-        if (BANDED) load_rotation(rec4, s.T);
-        const int Uv = oU + (src & (kBrick - 1)), Vv = oV + warp + 8 * (src >> 4);
-        const int X = AX::W == 0 ? wv : (AX::U == 0 ? Uv : Vv);
-        const int Y = AX::W == 1 ? wv : (AX::U == 1 ? Uv : Vv);
-        const int Z = AX::W == 2 ? wv : Vv;
-        float re, im, w;
-        bool ok;
-        if (FAST)
-          ok = voxel_nearest<STORAGE, BANDED>(G, s, img, bandStride, scale, X, Y, Z, re, im, w);
-        else if (G.genericTaps)
-          ok = voxel_blob<MODE, TAPS, STORAGE, true, BANDED>(P, G, s, img, bandStride, scale, lut, X, Y, Z, re, im, w);
-        else
-          ok = voxel_blob<MODE, TAPS, STORAGE, false, BANDED>(P, G, s, img, bandStride, scale, lut, X, Y, Z, re, im, w);
-        if (ok) {
-          const int li = acc_index(X - ox, Y - oy, Z - oz);
-          acc_add<KAHAN>(A.re, A.cre, li, re);
-          acc_add<KAHAN>(A.im, A.cim, li, im);
-          acc_add<KAHAN>(A.w, A.cw, li, w);
+          for (int j = 0; j < 7; ++j) {
+            if (j < cnt) list[excl + j] = uint16_t(v);
+            v += col.sW;
+          }
+          have = total;
+          ++e;
+        } else {  // long columns, or more voxels than the list takes: in rounds
+          const unsigned c3 = __ballot_sync(0xffffffffu, cnt & 8), c4 = __ballot_sync(0xffffffffu, cnt & 16);
+          excl += 8 * __popc(c3 & before) + 16 * __popc(c4 & before);
+          total += 8 * __popc(c3) + 16 * __popc(c4);
+          have = min(total - listed, kVoxelList);
+          __syncwarp();
+          for (int j = 0; j < cnt; ++j, v += col.sW) {
+            const int k = excl + j - listed;
+            if (k >= 0 && k < have) list[k] = uint16_t(v);
+          }
+          listed += have;
+          if (listed == total) {
+            listed = 0;
+            ++e;
+          }
         }
+        __syncwarp();
+        at = 0;
+        continue;
       }
+      const int k = at + lane - n;
+      if (lane >= n && k < have) {
+        voxel = list[k] | parts << 12;
+        space = si;
+      }
+      const int took = min(32 - n, have - at);
+      at += took;
+      n += took;
+      ++parts;
     }
-    __syncwarp();  // the next projection may revisit these voxels from other lanes
+    if (n == 0) break;
+    float2 v;
+    float w;
+    bool ok = false;
+    if (lane < n) {
+      const VoxelRec s = load_voxel_rec(P.recs + space);
+      const float px = voxel_coord(voxel & 15, bx), py = voxel_coord(voxel >> 4 & 15, by),
+                  pz = voxel_coord(voxel >> 8 & 15, bz);
+      const float scale = STORAGE == FR_STORAGE_FP32 ? 1.f : __ldg(G.scales + s.proj);
+      const PT *img = reinterpret_cast<const PT *>(G.fft) + size_t(unsigned(s.proj)) * plane;
+      if (G.genericTaps)
+        ok = voxel_blob<MODE, TAPS, STORAGE, true, BANDED>(P, G, s, img, bandStride, scale, lut, px, py, pz, v, w);
+      else
+        ok = voxel_blob<MODE, TAPS, STORAGE, false, BANDED>(P, G, s, img, bandStride, scale, lut, px, py, pz, v, w);
+    }
+    const int slot = acc_slot(voxel & 4095);
+    for (int p = 0; p < parts; ++p) {
+      if (ok && voxel >> 12 == p) acc_add<KAHAN>(A, slot, v, w);
+      __syncwarp();  // the next entry or step may revisit these voxels from other lanes
+    }
+    n = 0;
+    parts = 0;
   }
+}
+
+// All list entries [e0, e1) of one direction, nearest-pixel insertion: at most one voxel per
+// column and projection, which the column's lane inserts itself (no lane touches another's column,
+// so no synchronisation either).
+template<int STORAGE, bool KAHAN, bool JOBS, bool BANDED>
+__device__ __forceinline__ void insert_nearest(const InsertParams &P, const JobGeom &G, const Accum &A, int ox,
+  int oy, int oz, int dir, int warp, int lane, int e0, int e1)
+{
+  using PT = typename Pixel<STORAGE>::T;
+  const int bandStride = JOBS ? G.bandStride : P.bandStride;
+  const size_t plane = BANDED ? size_t((G.fftY + 3) / 4) * size_t(bandStride) : size_t(G.fftX) * size_t(G.fftY);
+  const Column col = column_of(G, dir, ox, oy, oz, warp, lane);
+  const float bx = brick_origin(ox, G.cx), by = brick_origin(oy, G.cy), bz = brick_origin(oz, G.cz);
+  for (int e = col.in ? e0 : e1; e < e1; ++e) {
+    const int si = __ldg(P.list + e);
+    const float4 *q = reinterpret_cast<const float4 *>(P.recs + si);
+    const float4 box = __ldg(q + 3), n = __ldg(q + 6), b = __ldg(q + 7);
+    if (col.U < box.x || col.U > box.y || col.V < box.z || col.V > box.w) continue;
+    // the reference's rounded plane hit
+    const int W = int(add_(plane_hit(col.U, col.V, n.x, n.y, n.z, n.w, b.x, b.y), 0.5f));
+    if (W < col.oW || W > col.wHi) continue;
+    const int lin = col.lin + W * col.sW;
+    const VoxelRec s = load_voxel_rec(P.recs + si);
+    const float scale = STORAGE == FR_STORAGE_FP32 ? 1.f : __ldg(G.scales + s.proj);
+    const PT *img = reinterpret_cast<const PT *>(G.fft) + size_t(unsigned(s.proj)) * plane;
+    float2 v;
+    float w;
+    if (voxel_nearest<STORAGE, BANDED>(G, s, img, bandStride, scale, voxel_coord(lin & 15, bx),
+          voxel_coord(lin >> 4 & 15, by), voxel_coord(lin >> 8, bz), v, w))
+      acc_add<KAHAN>(A, acc_slot(lin), v, w);
+  }
+  __syncwarp();
 }
 
 // Shared-memory groups per CTA: one 256-thread group per brick in flight.  The groups of a CTA
@@ -444,6 +531,7 @@ __global__ void __launch_bounds__(kThreads *Groups<KAHAN>::value, 1) insert_kern
   extern __shared__ float4 smem4[];
   float *smem = reinterpret_cast<float *>(smem4);
   __shared__ int sItem[kMaxGroups];
+  __shared__ uint16_t sVoxels[FAST ? 1 : kMaxGroups * (kThreads / 32)][kVoxelList];
   // Batched launches: the current job's geometry, one copy per group in shared memory.  Held
   // in registers (as the single-job kernel may, where the values are constant operands of the
   // launch parameters) its 20 words spilled 80 bytes at the register cap.
@@ -453,12 +541,10 @@ __global__ void __launch_bounds__(kThreads *Groups<KAHAN>::value, 1) insert_kern
   const int warp = tid >> 5, lane = tid & 31;
   float *acc = smem + group * kAccFloats;
   Accum A;
-  A.re = acc;
-  A.im = acc + kBrickVox;
+  A.v = reinterpret_cast<float2 *>(acc);
   A.w = acc + 2 * kBrickVox;
-  A.cre = reinterpret_cast<__nv_bfloat16 *>(acc + 3 * kBrickVox);
-  A.cim = A.cre + kBrickVox;
-  A.cw = A.cim + kBrickVox;
+  A.cv = reinterpret_cast<__nv_bfloat162 *>(acc + 3 * kBrickVox);
+  A.cw = reinterpret_cast<__nv_bfloat16 *>(A.cv + kBrickVox);
   float *lutS = smem + nGroups * kAccFloats;
 
   const float *lut = P.table;
@@ -467,20 +553,22 @@ __global__ void __launch_bounds__(kThreads *Groups<KAHAN>::value, 1) insert_kern
     for (int i = threadIdx.x; i < nf; i += int(blockDim.x)) lutS[i] = __ldg(P.table + i);
     lut = lutS;
   }
+  for (int i = tid; i < kAccFloats; i += kThreads) acc[i] = 0.f;  // the flush leaves zeros behind
+  if (tid == 0) sItem[group] = atomicAdd(P.workCounter, 1);
   __syncthreads();
   const int nItems = *P.nItems;
 
   for (;;) {
-    group_sync(group);
-    if (tid == 0) sItem[group] = atomicAdd(P.workCounter, 1);
-    group_sync(group);
+    group_sync(group);  // the flush is finished, the next item's index is there
     const int itIdx = sItem[group];
     if (itIdx >= nItems) break;
     const WorkItem it = P.items[itIdx];
-    // (the group finished its previous item, flush included, before the barrier above)
-    if (JOBS && tid == 0) sGeom[group] = geom_of(P.jobs[it.job]);
-    for (int i = tid; i < kAccFloats; i += kThreads) acc[i] = 0.f;
-    group_sync(group);
+    int next = 0;  // fetched while this item is inserted
+    if (tid == 0) next = atomicAdd(P.workCounter, 1);
+    if (JOBS) {
+      if (tid == 0) sGeom[group] = geom_of(P.jobs[it.job]);
+      group_sync(group);
+    }
     JobGeom Gl;
     if (!JOBS) Gl = geom_of(P);
     const JobGeom &G = JOBS ? sGeom[group] : Gl;
@@ -493,34 +581,36 @@ __global__ void __launch_bounds__(kThreads *Groups<KAHAN>::value, 1) insert_kern
       const int e0 = max(it.begin, P.offsets[base + dir]);
       const int e1 = min(it.end, P.offsets[base + dir + 1]);
       if (e0 >= e1) continue;  // uniform across the group
-      if (dir == FR_DIR_XY)
-        run_direction<FR_DIR_XY, MODE, TAPS, FAST, STORAGE, KAHAN, JOBS, BANDED>(P, G, A, lut, ox, oy, oz, warp, lane,
-          e0, e1);
-      else if (dir == FR_DIR_XZ)
-        run_direction<FR_DIR_XZ, MODE, TAPS, FAST, STORAGE, KAHAN, JOBS, BANDED>(P, G, A, lut, ox, oy, oz, warp, lane,
-          e0, e1);
+      if (FAST)
+        insert_nearest<STORAGE, KAHAN, JOBS, BANDED>(P, G, A, ox, oy, oz, dir, warp, lane, e0, e1);
       else
-        run_direction<FR_DIR_YZ, MODE, TAPS, FAST, STORAGE, KAHAN, JOBS, BANDED>(P, G, A, lut, ox, oy, oz, warp, lane,
-          e0, e1);
+        insert_blobs<MODE, TAPS, STORAGE, KAHAN, JOBS, BANDED>(P, G, A, lut, sVoxels[threadIdx.x >> 5], ox, oy, oz, dir, warp, lane, e0, e1);
       group_sync(group);  // the next direction maps warps to other voxels
     }
-    // add the brick into the caller's volume
-    for (int li = tid; li < kBrickVox; li += kThreads) {
-      const int lz = li / (kBrick * kBrick), ly = (li / kBrick) & (kBrick - 1);
-      const int lx = (li & (kBrick - 1)) ^ ((lz + (ly >> 1)) & (kBrick - 1));
-      const int X = ox + lx, Y = oy + ly, Z = oz + lz;
-      if (X >= G.vx || Y >= G.vy || Z >= G.vz) continue;
-      float re = A.re[li], im = A.im[li], w = A.w[li];
+    // add the brick into the caller's volume and clear it (an item has at least one entry, so a
+    // barrier lies between the reads of sItem above and its new value)
+    for (int lin = tid; lin < kBrickVox; lin += kThreads) {
+      const int i = acc_slot(lin);
+      float2 v = A.v[i];
+      float w = A.w[i];
+      A.v[i] = make_float2(0.f, 0.f);
+      A.w[i] = 0.f;
       if (KAHAN) {
-        re = __fsub_rn(re, __bfloat162float(A.cre[li]));
-        im = __fsub_rn(im, __bfloat162float(A.cim[li]));
-        w = __fsub_rn(w, __bfloat162float(A.cw[li]));
+        const float2 c = __bfloat1622float2(A.cv[i]);
+        v.x = __fsub_rn(v.x, c.x);
+        v.y = __fsub_rn(v.y, c.y);
+        w = __fsub_rn(w, __bfloat162float(A.cw[i]));
+        A.cv[i] = __floats2bfloat162_rn(0.f, 0.f);
+        A.cw[i] = __float2bfloat16_rn(0.f);
       }
-      if (__float_as_uint(re) == 0u && __float_as_uint(im) == 0u && __float_as_uint(w) == 0u) continue;
+      const int X = ox + (lin & 15), Y = oy + (lin >> 4 & 15), Z = oz + (lin >> 8);
+      if (X >= G.vx || Y >= G.vy || Z >= G.vz) continue;
+      if (__float_as_uint(v.x) == 0u && __float_as_uint(v.y) == 0u && __float_as_uint(w) == 0u) continue;
       const size_t g = (size_t(Z) * G.vy + Y) * G.vx + X;
-      atomicAdd(reinterpret_cast<float2 *>(G.volume) + g, make_float2(re, im));
+      atomicAdd(reinterpret_cast<float2 *>(G.volume) + g, v);
       atomicAdd(G.weight + g, w);
     }
+    if (tid == 0) sItem[group] = next;
   }
 }
 

@@ -764,6 +764,10 @@ int insert_groups(const InsertConfig &cfg)
   return cfg.groups > 0 && cfg.groups < mx ? cfg.groups : mx;
 }
 
+// Static shared memory of the insertion kernel (at most): the voxel lists of its 24 warps and a
+// few words.
+constexpr size_t kInsertStaticSmem = 12 << 10;
+
 // Bytes of the kernel's table (the lookup table's entries, or the fixed Kaiser table of
 // dynamic interpolation); 0 when the mode reads none.
 static size_t table_bytes(const InsertConfig &cfg, int tableElems)
@@ -778,7 +782,7 @@ bool insert_lut_in_smem(const InsertConfig &cfg, int tableElems)
 {
   const size_t acc = size_t(insert_groups(cfg)) * size_t(cfg.kahan ? 18 : 12) * kBrickVox;
   const size_t t = table_bytes(cfg, tableElems);
-  return t > 0 && acc + t <= (227u << 10);
+  return t > 0 && acc + t + kInsertStaticSmem <= (227u << 10);
 }
 
 size_t insert_smem_bytes(const InsertConfig &cfg, int tableElems)
