@@ -231,11 +231,10 @@ typedef struct fr_prep_settings {
                                layout FR_LAYOUT_BANDED reads them in place); else row-major     */
 } fr_prep_settings;
 
-/* FR_PREP_FFT_FUSED: square images of side 64, 128 or 256 go through the engine's own FFT fused
- * with the processing (each image read once, each half-plane written once, the row spectra kept
- * in an L2-resident scratch); other sizes take the cuFFT route.  FR_PREP_FFT_CUFFT: cuFFT R2C
- * into a chunk of spectra, then one processing pass.  FR_PREP_FFT_AUTO (0, the default): the
- * fused route for FP32 output, the cuFFT route for 16-bit output. */
+/* FR_PREP_FFT_FUSED and FR_PREP_FFT_AUTO (0, the default): square images of side 64, 96, 128, 192,
+ * 256, 320 or 384 go through the engine's own FFT fused with the processing (spectra in an
+ * L2-resident scratch); other sizes take the cuFFT route.  FR_PREP_FFT_CUFFT: cuFFT R2C into a
+ * chunk of spectra, then one processing pass. */
 enum { FR_PREP_FFT_AUTO = 0, FR_PREP_FFT_CUFFT = 1, FR_PREP_FFT_FUSED = 2 };
 
 typedef struct fr_prep fr_prep;

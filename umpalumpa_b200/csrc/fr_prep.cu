@@ -1,8 +1,8 @@
 // Input preparation for insertion: real-to-complex FFT of the projection images and the
 // reference's Fourier processing -- crop, row shift, centring, normalisation, optional
 // frequency crop -- writing the half-planes in the layout fr_execute reads, optionally quantised
-// to 16 bits with a per-projection scale.  Square images of side 64, 128 or 256 go through the
-// engine's own FFT fused with the processing (fr_prep_fft.cuh); other sizes, or
+// to 16 bits with a per-projection scale.  Square images of side 64, 96, 128, 192, 256, 320 or 384
+// go through the engine's own FFT fused with the processing (fr_prep_fft.cuh); other sizes, or
 // FR_PREP_FFT_CUFFT, through cuFFT and one processing pass (below).  The C-ABI is declared in
 // include/umpalumpa_fr.h.
 //
@@ -165,7 +165,7 @@ struct fr_prep {
   cufftHandle plan = 0, tail = 0;
   int tail_batch = 0;
   float2 *spectra = nullptr;
-  // fused route: side N, one scratch of (N/2 + 1) x N per persistent CTA, the twiddle table
+  // fused route: side N, one scratch per persistent CTA, the twiddle table
   int fused = 0;
   int ctas = 0;
   float2 *scratch = nullptr;
@@ -174,43 +174,40 @@ struct fr_prep {
 
 namespace {
 
-// Side of the fused route for these settings (0: cuFFT route).  FR_PREP_FFT_AUTO takes the
-// fused route for FP32 output only: with 16-bit output its extra transpose pass through the
-// scratch made it slower than the cuFFT route (1.96 M against 2.49 M box-256 images/s on a
-// B200, FP32 2.95 M against 2.92 M).
+// Side of the fused route for these settings (0: cuFFT route).  It is the faster one at every side
+// and storage it covers (fr_prep_fft.cuh).
 int fused_side(const fr_prep_settings &s)
 {
   if (s.fft == FR_PREP_FFT_CUFFT || s.size_x != s.size_y) return 0;
-  if (s.fft == FR_PREP_FFT_AUTO && s.storage != FR_STORAGE_FP32) return 0;
-  return (s.size_x == 64 || s.size_x == 128 || s.size_x == 256) ? int(s.size_x) : 0;
+  switch (s.size_x) {
+  case 64: case 96: case 128: case 192: case 256: case 320: case 384: return int(s.size_x);
+  default: return 0;
+  }
 }
 
-template<int N> cudaError_t launch_fused(fr_prep *p, const frb::prepfft::Args &a)
+// Calls f with the fused route's shape of side n, at compile time.
+template<class F> cudaError_t with_side(int n, F f)
 {
-  const size_t smem = frb::prepfft::smem_bytes<N>();
-  const int grid = std::min(a.n, p->ctas);
-  cudaError_t e;
-  switch (p->s.storage) {
-  case FR_STORAGE_BF16:
-    e = cudaFuncSetAttribute(frb::prepfft::prep_fft_kernel<N, FR_STORAGE_BF16>,
-                             cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
-    if (e == cudaSuccess)
-      frb::prepfft::prep_fft_kernel<N, FR_STORAGE_BF16><<<grid, frb::prepfft::kThreads, smem, p->stream>>>(a);
-    break;
-  case FR_STORAGE_FP16:
-    e = cudaFuncSetAttribute(frb::prepfft::prep_fft_kernel<N, FR_STORAGE_FP16>,
-                             cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
-    if (e == cudaSuccess)
-      frb::prepfft::prep_fft_kernel<N, FR_STORAGE_FP16><<<grid, frb::prepfft::kThreads, smem, p->stream>>>(a);
-    break;
-  default:
-    e = cudaFuncSetAttribute(frb::prepfft::prep_fft_kernel<N, FR_STORAGE_FP32>,
-                             cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
-    if (e == cudaSuccess)
-      frb::prepfft::prep_fft_kernel<N, FR_STORAGE_FP32><<<grid, frb::prepfft::kThreads, smem, p->stream>>>(a);
-    break;
+  using namespace frb::prepfft;
+  switch (n) {
+  case 64: return f(Side<64>());
+  case 96: return f(Side<96>());
+  case 128: return f(Side<128>());
+  case 192: return f(Side<192>());
+  case 256: return f(Side<256>());
+  case 320: return f(Side<320>());
+  default: return f(Side<384>());
   }
-  return e == cudaSuccess ? cudaGetLastError() : e;
+}
+
+template<int N, int STORAGE, bool BANDED = false> cudaError_t launch_fused(fr_prep *p, const frb::prepfft::Args &a)
+{
+  using Sh = frb::prepfft::Shape<N>;
+  auto *kernel = frb::prepfft::prep_fft_kernel<N, STORAGE, BANDED>;
+  const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(Sh::smem));
+  if (e != cudaSuccess) return e;
+  kernel<<<std::min(a.n, p->ctas), Sh::threads, Sh::smem, p->stream>>>(a);
+  return cudaGetLastError();
 }
 
 }// namespace
@@ -275,17 +272,23 @@ int fr_prep_create(int device, void *stream, const fr_prep_settings *s, fr_prep 
   int rc = FR_OK;
   p->fused = fused_side(*s);
   if (p->fused) {
-    // persistent CTAs (kCtasPerSm per SM), each with its own column-major scratch of the row spectra
+    // persistent CTAs, each with its own scratch of the column spectra
     const int N = p->fused;
     int sms = 0;
     if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess) sms = 1;
-    p->ctas = std::max(1, sms) * frb::prepfft::kCtasPerSm;
-    std::vector<float2> tw(N);
+    size_t scratchBytes = 0;
+    with_side(N, [&](auto side) {
+      using Sh = frb::prepfft::Shape<decltype(side)::value>;
+      p->ctas = std::max(1, sms) * Sh::ctas;
+      scratchBytes = std::max<size_t>(1, size_t(p->ctas) * Sh::l2Rows * Sh::pitch) * sizeof(float2);
+      return cudaSuccess;
+    });
+    std::vector<float2> tw(N);  // [16][N / 16]: e^{-2 pi i j k1 / N}
     for (int t = 0; t < N; ++t) {
-      const double a = -2.0 * 3.14159265358979323846 * double(t) / double(N);
+      const int k1 = t / (N / 16), j = t % (N / 16);
+      const double a = -2.0 * 3.14159265358979323846 * double(j * k1) / double(N);
       tw[t] = make_float2(float(std::cos(a)), float(std::sin(a)));
     }
-    const size_t scratchBytes = size_t(p->ctas) * size_t(N / 2 + 1) * N * sizeof(float2);
     if (cudaMalloc(reinterpret_cast<void **>(&p->scratch), scratchBytes) != cudaSuccess
         || cudaMalloc(reinterpret_cast<void **>(&p->twiddles), N * sizeof(float2)) != cudaSuccess
         || cudaMemcpy(p->twiddles, tw.data(), N * sizeof(float2), cudaMemcpyHostToDevice) != cudaSuccess) {
@@ -342,9 +345,14 @@ int fr_prep_execute(fr_prep *p, const float *images, uint64_t n, void *out, floa
     f.scales = scales;
     f.bandStride = banded ? frb::band_stride(f.outX) : 0;
     f.outPlane = banded ? frb::band_plane_elems(f.outX, f.outY) : int64_t(f.outX) * f.outY;
-    cudaError_t e = p->fused == 256 ? launch_fused<256>(p, f)
-                    : p->fused == 128 ? launch_fused<128>(p, f)
-                                      : launch_fused<64>(p, f);
+    const cudaError_t e = with_side(p->fused, [&](auto side) {
+      constexpr int N = decltype(side)::value;
+      switch (p->s.storage) {
+      case FR_STORAGE_BF16: return launch_fused<N, FR_STORAGE_BF16>(p, f);
+      case FR_STORAGE_FP16: return launch_fused<N, FR_STORAGE_FP16>(p, f);
+      default: return banded ? launch_fused<N, FR_STORAGE_FP32, true>(p, f) : launch_fused<N, FR_STORAGE_FP32>(p, f);
+      }
+    });
     if (e != cudaSuccess) {
       cudaGetLastError();
       return fail(FR_E_CUDA, std::string("fused prep launch failed: ") + cudaGetErrorString(e));

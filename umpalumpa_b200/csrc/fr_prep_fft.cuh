@@ -1,25 +1,33 @@
-// Fused input preparation for square power-of-two images (N = 64, 128, 256): the real-to-complex
-// 2D FFT and the reference's Fourier processing in one kernel that reads each image once and
-// writes its finished half-plane once.
+// Fused input preparation for square images of side N = 64, 96, 128, 192, 256, 320 or 384: the
+// real-to-complex 2D FFT and the reference's Fourier processing in one kernel that reads each
+// image once and writes its finished half-plane once.
 //
 // The reference runs AFFT (batched cuFFT R2C, fourier_transformation/fft_cuda.cpp:92-95), whose
 // spectra go to a buffer, and AFP (scaleFFT2DKernel, fourier_processing/fp_cuda_kernels.cu:9-61),
-// which reads that buffer and writes a second one.  Here persistent CTAs (two per SM) take images
-// in turn:
-//   1. row pass: two image rows form one complex sequence z = a + ib; its N-point DFT Z gives
-//      both rows' half spectra, A[k] = (Z[k] + conj Z[N-k]) / 2 and B[k] = (Z[k] - conj Z[N-k]) / 2i,
-//      k = 0..N/2, staged in shared memory and written column-major to the CTA's own scratch
-//      (N/2+1 columns of N values, 264 KB at N = 256: two per SM stay in L2);
-//   2. column pass: every needed column x < out_x goes through an N-point DFT; its values are
-//      processed exactly like ScaleFFT2DCPU (fp_cpu_kernels.hpp:24-36, crop / normalise /
-//      centre / row shift, each product rounded separately) and written to the output rows
-//      through a shared-memory transpose -- FP32 directly; for 16-bit storage written back to the
-//      column's scratch slot while the largest |re|, |im| is reduced, then quantised exactly like
-//      fr_quantize_projections in a tiled transpose pass from the scratch.
-// An N-point DFT is done by a team of N/16 threads holding 16 points each: a 16-point DFT per
-// thread (radix 4 x 4), twiddles e^{-2 pi i j k1 / N} from a table built in double precision on the host, a
-// transpose through the team's shared buffer, and N/16-point DFTs over the other index
-// (Cooley-Tukey with n = j + (N/16) m, k = k1 + 16 k2).
+// which reads that buffer and writes a second one.  Here persistent CTAs take images in turn:
+//   1. column pass: two adjacent image columns form one complex sequence z_y = I[y][2m] + i I[y][2m+1]
+//      (one 8-byte load per point, 128 contiguous bytes per 16 lanes); its N-point DFT Z_m goes,
+//      row by row, to the CTA's own scratch S[ky][m] (N rows of N/2 values, read back from L2).
+//   2. row pass: the column spectra of row ky come out of the rows ky and N - ky of S,
+//      C_2m = (Z_m[ky] + conj Z_m[N - ky]) / 2, C_2m+1 = (Z_m[ky] - conj Z_m[N - ky]) / 2i, and
+//      their N-point DFT over x gives F[ky][kx] for all kx -- and with it, as the image is real,
+//      F[N - ky][kx] = conj F[ky][N - kx]: N/2 - 1 row DFTs yield both halves.  The rows 0 and N/2,
+//      whose column spectra are real, share one DFT (real and imaginary part) and are separated
+//      afterwards.  The values are processed exactly like ScaleFFT2DCPU (fp_cpu_kernels.hpp:24-36,
+//      crop / normalise / centre / row shift, each product rounded separately) and stored from the
+//      registers, in the order of lanes that fills the rows' or the bands' sectors.  For 16-bit
+//      storage they go back to S while the largest |re|, |im| is reduced, and a last pass quantises
+//      them exactly like fr_quantize_projections.
+// A DFT of N = 16 TT points is two steps with an exchange through shared memory between them
+// (n = j + TT q, k = k1 + 16 k2): 16-point DFTs over q, twiddles e^{-2 pi i j k1 / N} from a table
+// built in double precision on the host, TT-point DFTs over j.  A pass runs 16 DFTs.
+//
+// What bounds it: latency and instruction issue at the 16 warps per SM its registers allow (N = 256;
+// the HBM floor, one read and one write, is 80 ns per image).  Measured per image, FP32 / BF16
+// rows, against cuFFT and a processing pass: N = 64 13 / 19 (23 / 30) ns, 96 24 / 31 (78 / 90),
+// 128 39 / 59 (79 / 99), 192 103 / 128 (211 / 254), 256 189 / 251 (329 / 436), 320 343 / 475
+// (839 / 1010), 384 556 / 738 (1216 / 1474) -- and against the kernel before, which took row pairs first,
+// separated and staged them in shared memory with four barriers a pass, 355 ns at N = 256.
 #pragma once
 
 #include <cuda_bf16.h>
@@ -31,162 +39,150 @@
 namespace frb {
 namespace prepfft {
 
-constexpr int kThreads = 256;
-constexpr int kCtasPerSm = 2;
+// ---- small DFTs in registers ------------------------------------------------------------------
 
-// cos and sin of 2 pi t / 16, t = 0..7
-__device__ __constant__ float kCos16[8] = { 1.0f, 0.92387953251128674f, 0.70710678118654752f, 0.38268343236508977f,
-  0.0f, -0.38268343236508977f, -0.70710678118654752f, -0.92387953251128674f };
-__device__ __constant__ float kSin16[8] = { 0.0f, 0.38268343236508977f, 0.70710678118654752f, 0.92387953251128674f,
-  1.0f, 0.92387953251128674f, 0.70710678118654752f, 0.38268343236508977f };
-
-// Bit-reversed index of i among S = 4, 8 or 16 points.
-template<int S, int I> struct BitRev {
-  static constexpr int value = S == 4 ? ((I & 1) << 1 | (I >> 1 & 1))
-                               : S == 8 ? ((I & 1) << 2 | (I & 2) | (I >> 2 & 1))
-                                        : ((I & 1) << 3 | (I & 2) << 1 | (I >> 1 & 2) | (I >> 3 & 1));
-};
-
-template<int S, int I = 0> __device__ __forceinline__ void bitrev_permute(float2 (&v)[S])
+// cos and sin of 2 pi e / S at compile time: exact at the quarter turns, else the Taylor series
+// of the angle reduced to at most a quarter turn, in double.
+__host__ __device__ constexpr double series(double x, bool sine)
 {
-  if constexpr (I < S) {
-    constexpr int J = BitRev<S, I>::value;
-    if constexpr (J > I) {
-      const float2 t = v[I];
-      v[I] = v[J];
-      v[J] = t;
-    }
-    bitrev_permute<S, I + 1>(v);
+  double term = sine ? x : 1.0, sum = term;
+  for (int k = sine ? 3 : 2; k < 30; k += 2) {
+    term *= -x * x / double(k * (k - 1));
+    sum += term;
+  }
+  return sum;
+}
+
+__host__ __device__ constexpr double turn_cos(int e, int s)
+{
+  e %= s;
+  if (2 * e > s) e = s - e;                       // cos(-a) = cos a
+  if (4 * e > s) return -turn_cos(s - 2 * e, 2 * s);  // cos(pi - a) = -cos a
+  if (4 * e == s) return 0.0;
+  return series(6.283185307179586476925287 * double(e) / double(s), false);
+}
+
+__host__ __device__ constexpr double turn_sin(int e, int s)
+{
+  e %= s;
+  if (2 * e > s) return -turn_sin(s - e, s);
+  if (4 * e > s) return turn_sin(s - 2 * e, 2 * s);
+  if (4 * e == s) return 1.0;
+  return series(6.283185307179586476925287 * double(e) / double(s), true);
+}
+
+__device__ __forceinline__ float2 cadd(float2 a, float2 b) { return __fadd2_rn(a, b); }
+__device__ __forceinline__ float2 csub(float2 a, float2 b) { return __ffma2_rn(b, make_float2(-1.f, -1.f), a); }
+__device__ __forceinline__ float2 cmul(float2 a, float2 w)
+{
+  return make_float2(fmaf(a.x, w.x, -a.y * w.y), fmaf(a.x, w.y, a.y * w.x));
+}
+
+// a * e^{-2 pi i E / S}
+template<int E, int S> __device__ __forceinline__ float2 rotate(float2 a)
+{
+  constexpr int e = E % S;
+  if constexpr (e == 0) return a;
+  else if constexpr (4 * e == S) return make_float2(a.y, -a.x);
+  else if constexpr (2 * e == S) return make_float2(-a.x, -a.y);
+  else if constexpr (4 * e == 3 * S) return make_float2(-a.y, a.x);
+  else {
+    constexpr float c = float(turn_cos(e, S)), s = float(-turn_sin(e, S));
+    return make_float2(fmaf(a.x, c, -a.y * s), fmaf(a.x, s, a.y * c));
   }
 }
 
-// Forward DFT (e^{-2 pi i n k / S}) of S = 4, 8 or 16 points in registers, natural order in and
-// out: radix-2 decimation in time after a bit-reversed permutation.
-// One radix-2 stage of butterflies of span LEN (all indices compile-time).
-template<int S, int LEN> __device__ __forceinline__ void dft_stage(float2 (&v)[S])
+template<int S> __device__ __forceinline__ void dft(float2 (&v)[S]);
+
+// v[I] for compile-time loops
+template<int A, int B, int N2, int K1> __device__ __forceinline__ void twiddle_column(float2 (&u)[A])
 {
+  if constexpr (K1 < A) {
+    u[K1] = rotate<N2 * K1, A * B>(u[K1]);
+    twiddle_column<A, B, N2, K1 + 1>(u);
+  }
+}
+
+template<int A, int B, int N2> __device__ __forceinline__ void inner_dfts(float2 (&v)[A * B])
+{
+  if constexpr (N2 < B) {
+    float2 u[A];
 #pragma unroll
-  for (int i = 0; i < S; i += LEN) {
+    for (int n1 = 0; n1 < A; ++n1) u[n1] = v[B * n1 + N2];
+    dft<A>(u);
+    twiddle_column<A, B, N2, 1>(u);
 #pragma unroll
-    for (int k = 0; k < LEN / 2; ++k) {
-      const int t = k * (16 / LEN);  // e^{-2 pi i k / LEN} = e^{-2 pi i t / 16}
-      const float c = t == 0 ? 1.f : kCos16[t], s = t == 0 ? 0.f : kSin16[t];
-      const float2 a = v[i + k], b = v[i + k + LEN / 2];
-      const float2 tb = make_float2(fmaf(b.x, c, b.y * s), fmaf(b.y, c, -b.x * s));
-      v[i + k] = make_float2(a.x + tb.x, a.y + tb.y);
-      v[i + k + LEN / 2] = make_float2(a.x - tb.x, a.y - tb.y);
-    }
-  }
-  if constexpr (LEN < S) dft_stage<S, 2 * LEN>(v);
-}
-
-// 4-point forward DFT of v[o], v[o + s], v[o + 2s], v[o + 3s] in place.
-template<int O, int ST, int S> __device__ __forceinline__ void dft4(float2 (&v)[S])
-{
-  const float2 x0 = v[O], x1 = v[O + ST], x2 = v[O + 2 * ST], x3 = v[O + 3 * ST];
-  const float2 a0 = make_float2(x0.x + x2.x, x0.y + x2.y), a1 = make_float2(x0.x - x2.x, x0.y - x2.y);
-  const float2 b0 = make_float2(x1.x + x3.x, x1.y + x3.y), b1 = make_float2(x1.x - x3.x, x1.y - x3.y);
-  v[O] = make_float2(a0.x + b0.x, a0.y + b0.y);
-  v[O + 2 * ST] = make_float2(a0.x - b0.x, a0.y - b0.y);
-  v[O + ST] = make_float2(a1.x + b1.y, a1.y - b1.x);       // a1 - i b1
-  v[O + 3 * ST] = make_float2(a1.x - b1.y, a1.y + b1.x);   // a1 + i b1
-}
-
-// e^{-2 pi i e / 16} for a compile-time exponent e
-template<int E> __device__ __forceinline__ float2 w16()
-{
-  constexpr int e = E & 15;
-  if constexpr (e == 0) return make_float2(1.f, 0.f);
-  else if constexpr (e == 4) return make_float2(0.f, -1.f);
-  else if constexpr (e == 8) return make_float2(-1.f, 0.f);
-  else if constexpr (e == 12) return make_float2(0.f, 1.f);
-  else if constexpr (e < 8) return make_float2(kCos16[e], -kSin16[e]);
-  else return make_float2(-kCos16[e - 8], kSin16[e - 8]);
-}
-
-template<int N2, int K1> __device__ __forceinline__ void twiddle16(float2 (&v)[16])
-{
-  if constexpr (N2 * K1 != 0) {
-    const float2 w = w16<N2 * K1>();
-    const float2 a = v[4 * K1 + N2];
-    v[4 * K1 + N2] = make_float2(fmaf(a.x, w.x, -a.y * w.y), fmaf(a.x, w.y, a.y * w.x));
+    for (int k1 = 0; k1 < A; ++k1) v[B * k1 + N2] = u[k1];
+    inner_dfts<A, B, N2 + 1>(v);
   }
 }
 
-// Forward DFT (e^{-2 pi i n k / S}) of S = 4, 8 or 16 points in registers, natural order in and
-// out.  16 points: radix 4 x 4 (n = 4 n1 + n2, k = k1 + 4 k2); 8: radix 2 after a bit-reversed
-// permutation; 4: one radix-4 butterfly.
+// A x B points, n = B n1 + n2, k = k1 + A k2: A-point DFTs over n1, twiddles, B-point DFTs over n2.
+template<int A, int B> __device__ __forceinline__ void composite(float2 (&v)[A * B])
+{
+  inner_dfts<A, B, 0>(v);
+  float2 o[A * B];
+#pragma unroll
+  for (int k1 = 0; k1 < A; ++k1) {
+    float2 u[B];
+#pragma unroll
+    for (int n2 = 0; n2 < B; ++n2) u[n2] = v[B * k1 + n2];
+    dft<B>(u);
+#pragma unroll
+    for (int k2 = 0; k2 < B; ++k2) o[k1 + A * k2] = u[k2];
+  }
+#pragma unroll
+  for (int k = 0; k < A * B; ++k) v[k] = o[k];
+}
+
+// Forward DFT (e^{-2 pi i n k / S}) of S points in registers, natural order in and out.
 template<int S> __device__ __forceinline__ void dft(float2 (&v)[S])
 {
-  static_assert(S == 4 || S == 8 || S == 16, "4, 8 or 16 points");
-  if constexpr (S == 4) {
-    dft4<0, 1>(v);
-  } else if constexpr (S == 8) {
-    bitrev_permute<S>(v);
-    dft_stage<S, 2>(v);
+  if constexpr (S == 2) {
+    const float2 a = v[0], b = v[1];
+    v[0] = cadd(a, b);
+    v[1] = csub(a, b);
+  } else if constexpr (S == 3) {
+    constexpr float h = float(turn_sin(1, 3));
+    const float2 t = cadd(v[1], v[2]), d = csub(v[1], v[2]);
+    const float2 m = __ffma2_rn(t, make_float2(-0.5f, -0.5f), v[0]);
+    v[0] = cadd(v[0], t);
+    v[1] = make_float2(fmaf(h, d.y, m.x), fmaf(-h, d.x, m.y));
+    v[2] = make_float2(fmaf(-h, d.y, m.x), fmaf(h, d.x, m.y));
+  } else if constexpr (S == 4) {
+    const float2 a0 = cadd(v[0], v[2]), a1 = csub(v[0], v[2]), b0 = cadd(v[1], v[3]), b1 = csub(v[1], v[3]);
+    v[0] = cadd(a0, b0);
+    v[2] = csub(a0, b0);
+    v[1] = make_float2(a1.x + b1.y, a1.y - b1.x);  // a1 - i b1
+    v[3] = make_float2(a1.x - b1.y, a1.y + b1.x);  // a1 + i b1
+  } else if constexpr (S == 5) {
+    constexpr float c1 = float(turn_cos(1, 5)), c2 = float(turn_cos(2, 5));
+    constexpr float s1 = float(turn_sin(1, 5)), s2 = float(turn_sin(2, 5));
+    const float2 t1 = cadd(v[1], v[4]), t2 = cadd(v[2], v[3]), d1 = csub(v[1], v[4]), d2 = csub(v[2], v[3]);
+    const float2 m1 = __ffma2_rn(t2, make_float2(c2, c2), __ffma2_rn(t1, make_float2(c1, c1), v[0]));
+    const float2 m2 = __ffma2_rn(t2, make_float2(c1, c1), __ffma2_rn(t1, make_float2(c2, c2), v[0]));
+    const float2 n1 = __ffma2_rn(d2, make_float2(s2, s2), __fmul2_rn(d1, make_float2(s1, s1)));
+    const float2 n2 = __ffma2_rn(d2, make_float2(-s1, -s1), __fmul2_rn(d1, make_float2(s2, s2)));
+    v[0] = cadd(v[0], cadd(t1, t2));
+    v[1] = make_float2(m1.x + n1.y, m1.y - n1.x);
+    v[4] = make_float2(m1.x - n1.y, m1.y + n1.x);
+    v[2] = make_float2(m2.x + n2.y, m2.y - n2.x);
+    v[3] = make_float2(m2.x - n2.y, m2.y + n2.x);
+  } else if constexpr (S % 4 == 0) {
+    composite<4, S / 4>(v);
   } else {
-    // 4-point DFTs over n1 for each n2: x[4 n1 + n2] -> Y[n2][k1] held at v[4 k1 + n2]
-    dft4<0, 4>(v);
-    dft4<1, 4>(v);
-    dft4<2, 4>(v);
-    dft4<3, 4>(v);
-    // twiddles e^{-2 pi i n2 k1 / 16}
-    twiddle16<1, 1>(v); twiddle16<1, 2>(v); twiddle16<1, 3>(v);
-    twiddle16<2, 1>(v); twiddle16<2, 2>(v); twiddle16<2, 3>(v);
-    twiddle16<3, 1>(v); twiddle16<3, 2>(v); twiddle16<3, 3>(v);
-    // 4-point DFTs over n2 for each k1: v[4 k1 + n2] -> X[k1 + 4 k2] at v[4 k1 + k2]
-    dft4<0, 1>(v);
-    dft4<4, 1>(v);
-    dft4<8, 1>(v);
-    dft4<12, 1>(v);
-    // transpose the 4 x 4 index: X[k1 + 4 k2] sits at v[4 k1 + k2]
-    float2 t[16];
-#pragma unroll
-    for (int i = 0; i < 16; ++i) t[i] = v[i];
-#pragma unroll
-    for (int k1 = 0; k1 < 4; ++k1)
-#pragma unroll
-      for (int k2 = 0; k2 < 4; ++k2) v[k1 + 4 * k2] = t[4 * k1 + k2];
+    static_assert(S == 6, "2, 3, 4, 5, 6 or a multiple of 4 points");
+    composite<2, 3>(v);
   }
 }
 
-// N-point forward DFT by a team of TT = N / 16 lanes (lane j of the team holds x[j + TT m] in
-// v[m]); leaves Z[k] in natural order in buf[0..N) (the team's shared buffer of 16 x (TT + 1)
-// float2).  tw[t] = e^{-2 pi i t / N}.  Every lane of the warp calls it (teams tile the warp).
-template<int N> __device__ __forceinline__ void team_dft(float2 (&v)[16], int j, float2 *buf, const float2 *tw)
-{
-  constexpr int TT = N / 16, P = TT + 1;
-  dft<16>(v);
-#pragma unroll
-  for (int k1 = 1; k1 < 16; ++k1) {
-    const float2 w = tw[j * k1];  // j k1 < TT * 16 = N
-    const float2 a = v[k1];
-    v[k1] = make_float2(fmaf(a.x, w.x, -a.y * w.y), fmaf(a.x, w.y, a.y * w.x));
-  }
-#pragma unroll
-  for (int k1 = 0; k1 < 16; ++k1) buf[k1 * P + j] = v[k1];
-  __syncwarp();
-  constexpr int Q = 16 / TT;  // k1 values per lane: k1 = j + TT q
-  float2 o[Q][TT];
-#pragma unroll
-  for (int q = 0; q < Q; ++q) {
-#pragma unroll
-    for (int jj = 0; jj < TT; ++jj) o[q][jj] = buf[(j + TT * q) * P + jj];
-    dft<TT>(o[q]);
-  }
-  __syncwarp();
-#pragma unroll
-  for (int q = 0; q < Q; ++q)
-#pragma unroll
-    for (int k2 = 0; k2 < TT; ++k2) buf[(j + TT * q) + 16 * k2] = o[q][k2];
-  __syncwarp();
-}
+// ---- the kernel -------------------------------------------------------------------------------
 
 struct Args {
   const float *images;   // [n][N][N]
   int n;
-  float2 *scratch;       // per CTA: [N/2 + 1][N]
-  const float2 *tw;      // [N]
+  float2 *scratch;       // per CTA: [l2Rows][pitch]
+  const float2 *tw;      // [16][N / 16]: e^{-2 pi i j k1 / N}
   int outX, outY;
   int normalize, center, shift, crop;
   float maxFreq, norm;
@@ -204,145 +200,225 @@ __device__ __forceinline__ float idx2freq_(int idx, int size)
   return __fdiv_rn(t, float(size));
 }
 
-template<int N> __host__ __device__ constexpr size_t smem_bytes()
-{
-  // twiddles + team buffers + the staging area (row pass [rows][N/2+1], column pass [N][teams],
-  // 16-bit transpose tiles)
-  constexpr int TT = N / 16, TEAMS = kThreads / TT;
-  constexpr int rows = 2 * TEAMS < N ? 2 * TEAMS : N;
-  constexpr size_t rowStage = size_t(rows) * (N / 2 + 1);
-  constexpr size_t colStage = size_t(N) * TEAMS;
-  constexpr size_t stage = rowStage > colStage ? rowStage : colStage;
-  return (size_t(N) + size_t(TEAMS) * 16 * (TT + 1) + (stage > 32 * 33 ? stage : 32 * 33)) * sizeof(float2) + 64;
-}
+template<int N> struct Side { static constexpr int value = N; };
 
-template<int N, int STORAGE> __global__ void __launch_bounds__(kThreads, kCtasPerSm) prep_fft_kernel(Args a)
+template<int N> struct Shape {
+  static constexpr int TT = N / 16;
+  static constexpr int threads = 16 * (TT > 16 ? TT : 16);  // both steps of a pass in one go
+  static constexpr int pitch = N / 2 + 4;                   // scratch row (16-bit storage: N/2 + 1 values)
+  static constexpr int rowBuf = 16 * (TT + 1) + 4;          // exchange of one row DFT: 4 rows x 4 lanes conflict-free
+  static constexpr int buf = 16 * (rowBuf > 16 * TT ? rowBuf : 16 * TT);
+  static constexpr int ctas = N <= 64 ? 6 : N <= 128 ? 4 : N <= 192 ? 3 : N <= 256 ? 2 : 1;  // per SM
+  // The first rows of S, sixteen at a time, live in the shared memory the exchange leaves free
+  // under a carve-out of 164 KB; the rest of S, of all CTAs, has to stay in L2 beside the images
+  // that stream through.  N = 256: 189 ns per image, 202 with all rows in L2, 200 with a carve-out of
+  // 228 KB, whose L1 is too small for the row pass.
+  static constexpr int room = 164 * 1024 / ctas - 1024 - 128 - int((N + buf + N) * sizeof(float2));
+  static constexpr int fit = room > 0 ? room / int(16 * pitch * sizeof(float2)) : 0;
+  static constexpr int smemRows = 16 * (fit < TT ? fit : TT);
+  static constexpr int l2Rows = N - smemRows;
+  static constexpr size_t smem = (size_t(N + buf + N) + size_t(smemRows) * pitch) * sizeof(float2);
+  // Whether the next columns' points are loaded during a pass: they fit the registers beside it
+  // (128 and more per thread) from N = 256 on (208 -> 189 ns); below, they spill or cost a CTA
+  // (N = 128: 39 -> 47 ns).
+  static constexpr bool ahead = N >= 256;
+};
+
+// BANDED: FP32 output in bands (16-bit output takes its layout in the last pass).
+template<int N, int STORAGE, bool BANDED>
+__global__ void __launch_bounds__(Shape<N>::threads, Shape<N>::ctas) prep_fft_kernel(Args a)
 {
-  constexpr int TT = N / 16, P = TT + 1, TEAMS = kThreads / TT, H = N / 2 + 1;
-  constexpr int ROWS = 2 * TEAMS < N ? 2 * TEAMS : N;  // image rows per row pass
+  using Sh = Shape<N>;
+  constexpr int TT = Sh::TT, H = N / 2;
   extern __shared__ float2 sm[];
-  float2 *tw = sm;
-  float2 *teamBuf = tw + N;
-  float2 *stage = teamBuf + TEAMS * 16 * P;
-  __shared__ float red[kThreads / 32];
-  const int tid = threadIdx.x, team = tid / TT, j = tid % TT;
-  float2 *buf = teamBuf + team * 16 * P;
-  for (int i = tid; i < N; i += kThreads) tw[i] = a.tw[i];
-  float2 *S = a.scratch + size_t(blockIdx.x) * H * N;  // [H][N], column-major
+  float2 *tw = sm;            // [16][TT]
+  float2 *buf = tw + N;
+  float2 *edge = buf + Sh::buf;  // the DFT shared by the rows 0 and N/2
+  float2 *near = edge + N;       // rows of S in shared memory, the others in L2
+  __shared__ float red[Sh::threads / 32];
+  const int tid = threadIdx.x;
+  for (int i = tid; i < N; i += Sh::threads) tw[i] = a.tw[i];
+  float2 *far = a.scratch + size_t(blockIdx.x) * Sh::l2Rows * Sh::pitch;
+  auto S = [&](int row) -> float2 * {
+    return row < Sh::smemRows ? near + row * Sh::pitch : far + size_t(row - Sh::smemRows) * Sh::pitch;
+  };
+  const bool pairs = (reinterpret_cast<uintptr_t>(a.images) & 7) == 0;
   __syncthreads();
 
   for (int img = blockIdx.x; img < a.n; img += gridDim.x) {
     const float *I = a.images + size_t(img) * N * N;
-    // ---- 1. row pass: pairs of rows -> half spectra, staged, then written column-major
-    for (int y0 = 0; y0 < N; y0 += ROWS) {
-      const int r0 = min(2 * team, ROWS - 2);  // teams beyond the pass compute a row pair again
-      const float *ra = I + size_t(y0 + r0) * N, *rb = ra + N;
-      float2 v[16];
+    // ---- 1. column pass, 16 column pairs at a time, the next ones' points in flight
+    const int m = tid & 15, cj = tid >> 4;
+    float2 v[16];
+    auto load_columns = [&](int m0) {
+      const float *p = I + size_t(cj) * N + 2 * (m0 + m);
+      if (pairs) {
 #pragma unroll
-      for (int m = 0; m < 16; ++m) v[m] = make_float2(__ldg(ra + j + TT * m), __ldg(rb + j + TT * m));
-      team_dft<N>(v, j, buf, tw);
-      if (2 * team < ROWS) {
-        for (int k = j; k < H; k += TT) {
-          const float2 z = buf[k], zr = buf[(N - k) & (N - 1)];
-          stage[(2 * team) * H + k] = make_float2(0.5f * (z.x + zr.x), 0.5f * (z.y - zr.y));
-          stage[(2 * team + 1) * H + k] = make_float2(0.5f * (z.y + zr.y), -0.5f * (z.x - zr.x));
+        for (int q = 0; q < 16; ++q) v[q] = __ldcs(reinterpret_cast<const float2 *>(p + size_t(TT * q) * N));
+      } else {
+#pragma unroll
+        for (int q = 0; q < 16; ++q)
+          v[q] = make_float2(__ldcs(p + size_t(TT * q) * N), __ldcs(p + size_t(TT * q) * N + 1));
+      }
+    };
+    if (Sh::ahead && cj < TT) load_columns(0);
+    for (int m0 = 0; m0 < H; m0 += 16) {
+      if (cj < TT) {
+        if (!Sh::ahead) load_columns(m0);
+        dft<16>(v);
+#pragma unroll
+        for (int k1 = 0; k1 < 16; ++k1)
+          buf[(k1 * TT + cj) * 16 + m] = k1 ? cmul(v[k1], tw[k1 * TT + cj]) : v[0];
+        if (Sh::ahead && m0 + 16 < H) load_columns(m0 + 16);
+      }
+      __syncthreads();
+      if (tid < 256) {
+        const int k1 = cj;
+        float2 u[TT];
+#pragma unroll
+        for (int i = 0; i < TT; ++i) u[i] = buf[(k1 * TT + i) * 16 + m];
+        dft<TT>(u);
+#pragma unroll
+        for (int k2 = 0; k2 < TT; ++k2) {
+          if (16 * k2 < Sh::smemRows) near[(k1 + 16 * k2) * Sh::pitch + m0 + m] = u[k2];
+          else far[(k1 + 16 * k2 - Sh::smemRows) * Sh::pitch + m0 + m] = u[k2];
         }
       }
       __syncthreads();
-      for (int i = tid; i < ROWS * H; i += kThreads) {
-        const int k = i / ROWS, r = i - k * ROWS;
-        S[size_t(k) * N + y0 + r] = stage[r * H + k];
-      }
-      __syncthreads();
     }
-    // ---- 2. column pass
+    // the first columns of the CTA's next image, on their way to L2 during the row pass
+    if (img + int(gridDim.x) < a.n && tid < N)
+      asm volatile("prefetch.global.L2 [%0];" ::"l"(I + size_t(gridDim.x) * N * N + size_t(tid) * N));
+    // ---- 2. row pass, 16 rows ky (with their mirrors N - ky) at a time
     float amax = 0.f;
-    for (int x0 = 0; x0 < a.outX; x0 += TEAMS) {
-      const int x = min(x0 + team, a.outX - 1);  // teams beyond the last column repeat it
-      const bool live = x0 + team < a.outX;
-      float2 v[16];
-#pragma unroll
-      for (int m = 0; m < 16; ++m) v[m] = S[size_t(x) * N + j + TT * m];
-      team_dft<N>(v, j, buf, tw);
-      // ScaleFFT2DCPU on column x (fp_cpu_kernels.hpp:24-36)
-      for (int y = j; y < a.outY; y += TT) {
-        const int origY = y <= a.outY / 2 ? y : N - (a.outY - y);
-        float2 w = buf[origY];
-        if (a.crop) {
-          const float fx = idx2freq_(x, N), fy = idx2freq_(origY, N);
-          if (__fadd_rn(__fmul_rn(fx, fx), __fmul_rn(fy, fy)) > a.maxFreq) w = make_float2(0.f, 0.f);
-        }
-        if (a.normalize) w = make_float2(__fmul_rn(w.x, a.norm), __fmul_rn(w.y, a.norm));
-        if (a.center) {
-          const float c = float(1 - 2 * ((x + y) & 1));
-          w = make_float2(__fmul_rn(w.x, c), __fmul_rn(w.y, c));
-        }
-        const int t = y + a.outY / 2;
-        const int row = a.shift ? (t >= a.outY ? t - a.outY : t) : y;
-        if (STORAGE == FR_STORAGE_FP32) {
-          stage[row * TEAMS + team] = w;
-        } else if (live) {
-          amax = fmaxf(amax, fmaxf(fabsf(w.x), fabsf(w.y)));
-          S[size_t(x) * N + row] = w;  // the column was read whole above (v, then buf)
-        }
-      }
+    // The processed value F[origY][x] (twice: the separations leave their halves out) of output
+    // row y goes to element x of row_start(y, origY): ScaleFFT2DCPU's normalisation and centring
+    // are one product -- the halves and signs are exact -- whose factor is the same for all of a
+    // thread's values of a row and its mirror (x and y keep their parities).
+    constexpr int kStep = BANDED ? 4 : 1;
+    float2 *const O = static_cast<float2 *>(a.out) + size_t(img) * a.outPlane;
+    auto row_start = [&](int y, int origY) -> float2 * {
+      if (STORAGE != FR_STORAGE_FP32) return S(origY);  // its column spectra have been read whole
+      const int t = y + a.outY / 2;
+      const int row = a.shift ? (t >= a.outY ? t - a.outY : t) : y;
+      return BANDED ? O + size_t(row >> 2) * a.bandStride + (row & 3) : O + size_t(row) * a.outX;
+    };
+    auto factor_of = [&](int x, int y) {
+      const float f = a.normalize ? 0.5f * a.norm : 0.5f;
+      return a.center && ((x + y) & 1) ? -f : f;
+    };
+    auto cropped = [&](int x, int origY) {
+      const float fx = idx2freq_(x, N), fy = idx2freq_(origY, N);
+      return __fadd_rn(__fmul_rn(fx, fx), __fmul_rn(fy, fy)) > a.maxFreq;
+    };
+    auto emit = [&](float2 w, float f, float2 *row, int origY, int x) {
+      if (a.crop && cropped(x, origY)) w = make_float2(0.f, 0.f);
+      w = make_float2(w.x * f, w.y * f);
       if (STORAGE == FR_STORAGE_FP32) {
-        __syncthreads();
-        const int cols = min(TEAMS, a.outX - x0);
-        float2 *O = static_cast<float2 *>(a.out) + size_t(img) * a.outPlane;
-        if (a.bandStride) {  // (band, column, row within the band): contiguous runs of 4 cols
-          for (int i = tid; i < (a.outY + 3) / 4 * 4 * cols; i += kThreads) {
-            const int b = i / (4 * cols), r = i - b * 4 * cols, c = r >> 2, row = 4 * b + (r & 3);
-            if (row < a.outY) O[size_t(b) * a.bandStride + 4 * (x0 + c) + (row & 3)] = stage[row * TEAMS + c];
+        __stcs(row + kStep * x, w);
+      } else {
+        amax = fmaxf(amax, fmaxf(fabsf(w.x), fabsf(w.y)));
+        row[x] = w;
+      }
+    };
+    const int half = a.outY / 2;  // rows 0..half and N - (half - 1)..N - 1 are wanted
+    for (int r0 = 0; r0 < H && r0 <= half; r0 += 16) {
+      {
+        const int r = tid / TT, j = tid - r * TT, ky = r0 + r;
+        if (r < 16) {
+          float2 v[16];
+          const float2 *za = S(ky) + (j >> 1), *zb = S(ky ? N - ky : H) + (j >> 1);
+          const bool odd = j & 1;  // x = j + TT q, TT even
+#pragma unroll
+          for (int q = 0; q < 16; ++q) {
+            const float2 A = za[(TT / 2) * q], B = zb[(TT / 2) * q];
+            if (ky == 0) v[q] = odd ? make_float2(A.y, B.y) : make_float2(A.x, B.x);
+            else v[q] = odd ? make_float2(A.y + B.y, B.x - A.x) : make_float2(A.x + B.x, A.y - B.y);
           }
-        } else {
-          for (int i = tid; i < a.outY * cols; i += kThreads) {
-            const int row = i / cols, c = i - row * cols;
-            O[size_t(row) * a.outX + x0 + c] = stage[row * TEAMS + c];
-          }
+          dft<16>(v);
+#pragma unroll
+          for (int k1 = 0; k1 < 16; ++k1)
+            buf[r * Sh::rowBuf + k1 * (TT + 1) + j] = k1 ? cmul(v[k1], tw[k1 * TT + j]) : v[0];
         }
       }
       __syncthreads();
-    }
-    if (STORAGE != FR_STORAGE_FP32) {
-      // the image's largest |re|, |im|, then the quantised rows from the scratch by 32 x 32 tiles
-      for (int s = 16; s > 0; s >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, s));
-      if ((tid & 31) == 0) red[tid >> 5] = amax;
-      __syncthreads();
-      if (tid < 32) {
-        float m = tid < kThreads / 32 ? red[tid] : 0.f;
-        for (int s = 16; s > 0; s >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, s));
-        if (tid == 0) red[0] = m;
-      }
-      __syncthreads();
-      const float scale = red[0] > 0.f ? red[0] / 16384.f : 1.f;
-      const float inv = 1.f / scale;
-      if (tid == 0) a.scales[img] = scale;
-      float2 *tile = stage;  // [32][33]
-      for (int xb = 0; xb < a.outX; xb += 32)
-        for (int yb = 0; yb < a.outY; yb += 32) {
-          __syncthreads();
-          for (int i = tid; i < 32 * 32; i += kThreads) {
-            const int c = i / 32, r = i - c * 32;  // read down columns (contiguous rows)
-            if (xb + c < a.outX && yb + r < a.outY) tile[c * 33 + r] = S[size_t(xb + c) * N + yb + r];
+      if (tid < 256) {
+        // lanes: four rows x eight k1, so that eight columns of a band are stored whole
+        const int r = (tid & 3) | (tid >> 6) << 2, k1 = (tid >> 2) & 15, ky = r0 + r;
+        float2 u[TT];
+#pragma unroll
+        for (int i = 0; i < TT; ++i) u[i] = buf[r * Sh::rowBuf + k1 * (TT + 1) + i];
+        dft<TT>(u);
+        if (ky == 0) {
+#pragma unroll
+          for (int k2 = 0; k2 < TT; ++k2) edge[k1 + 16 * k2] = u[k2];
+        } else {
+          // columns kx <= N/2 of row ky, and of its mirror from kx >= N/2 (and 0)
+          const float f = factor_of(k1, ky);
+          float2 *const low = row_start(ky, ky), *const high = row_start(a.outY - ky, N - ky);
+          if (ky <= half) {
+#pragma unroll
+            for (int k2 = 0; k2 <= TT / 2; ++k2) {
+              const int x = k1 + 16 * k2;
+              if (x <= H && x < a.outX) emit(u[k2], f, low, ky, x);
+            }
           }
-          __syncthreads();
-          for (int i = tid; i < 32 * 32; i += kThreads) {
-            // write along rows, or banded: (band, column, row within the band)
-            const int r = a.bandStride ? 4 * (i >> 7) + (i & 3) : i / 32;
-            const int c = a.bandStride ? (i >> 2) & 31 : i - r * 32;
-            if (xb + c < a.outX && yb + r < a.outY) {
-              const float2 w = tile[c * 33 + r];
-              const int y = yb + r, x = xb + c;
-              const size_t d = size_t(img) * a.outPlane
-                               + (a.bandStride ? size_t(y >> 2) * a.bandStride + 4 * x + (y & 3) : size_t(y) * a.outX + x);
-              if (STORAGE == FR_STORAGE_BF16)
-                static_cast<__nv_bfloat162 *>(a.out)[d] = __floats2bfloat162_rn(w.x * inv, w.y * inv);
-              else
-                static_cast<__half2 *>(a.out)[d] = __floats2half2_rn(w.x * inv, w.y * inv);
+          if (ky < half) {
+#pragma unroll
+            for (int k2 = 0; k2 < TT; ++k2) {
+              if (k2 > 0 && k2 < TT / 2) continue;
+              const int kx = k1 + 16 * k2, x = kx ? N - kx : 0;
+              if (x <= H && x < a.outX) emit(make_float2(u[k2].x, -u[k2].y), f, high, N - ky, x);
             }
           }
         }
+      }
+      __syncthreads();
+      if (r0 == 0) {  // rows 0 and N/2 out of their common DFT
+        for (int x = tid; x < a.outX; x += Sh::threads) {
+          const float2 z = edge[x], zr = edge[x ? N - x : 0];
+          emit(make_float2(z.x + zr.x, z.y - zr.y), factor_of(x, 0), row_start(0, 0), 0, x);
+          if (half == H) emit(make_float2(z.y + zr.y, zr.x - z.x), factor_of(x, H), row_start(H, H), H, x);
+        }
+      }
+    }
+    if (STORAGE != FR_STORAGE_FP32) {
+      for (int s = 16; s > 0; s >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, s));
+      if ((tid & 31) == 0) red[tid >> 5] = amax;
+      __syncthreads();
+      float m = 0.f;
+      for (int w = 0; w < Sh::threads / 32; ++w) m = fmaxf(m, red[w]);
+      const float scale = m > 0.f ? m / 16384.f : 1.f;
+      const float inv = 1.f / scale;
+      if (tid == 0) a.scales[img] = scale;
+      // four output rows at a time, eight loads in flight: a warp stores 2 x 32 columns of each
+      // (rows) or of the band
+      const int bands = (a.outY + 3) / 4, tiles = (a.outX + 63) / 64;
+      const size_t base = size_t(img) * a.outPlane;
+      for (int t = tid >> 5; t < bands * tiles; t += Sh::threads / 32) {
+        const int b = t / tiles, x0 = 64 * (t - b * tiles) + (tid & 31);
+        float2 w[2][4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const int row = min(4 * b + i, a.outY - 1);
+          const int y = a.shift ? (row >= half ? row - half : row + half) : row;
+          const float2 *src = S(y <= half ? y : N - (a.outY - y));
+#pragma unroll
+          for (int h = 0; h < 2; ++h) w[h][i] = src[min(x0 + 32 * h, a.outX - 1)];
+        }
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            const int row = 4 * b + i, x = x0 + 32 * h;
+            if (x >= a.outX || row >= a.outY) continue;
+            const size_t d = base + (a.bandStride ? size_t(b) * a.bandStride + 4 * x + i : size_t(row) * a.outX + x);
+            if (STORAGE == FR_STORAGE_BF16)
+              static_cast<__nv_bfloat162 *>(a.out)[d] = __floats2bfloat162_rn(w[h][i].x * inv, w[h][i].y * inv);
+            else
+              static_cast<__half2 *>(a.out)[d] = __floats2half2_rn(w[h][i].x * inv, w[h][i].y * inv);
+          }
+      }
       __syncthreads();
     }
   }

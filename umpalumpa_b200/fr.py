@@ -530,9 +530,9 @@ class Prep:
 
     Defaults are the settings the example driver uses (normalise, centre, shift; no frequency
     crop, examples/fourier_reconstruction/fr.cpp:166-204) and the full half-plane.  fft="fused"
-    runs square images of side 64, 128 or 256 through the engine's own FFT fused with the
-    processing (other sizes through cuFFT); fft="cufft" always takes the cuFFT route; "auto"
-    fuses for FP32 output only.  layout="banded" writes the half-planes in the insertion's banded
+    and "auto" run square images of side 64, 96, 128, 192, 256, 320 or 384 through the engine's
+    own FFT fused with the processing (other sizes through cuFFT); fft="cufft" always takes the
+    cuFFT route.  layout="banded" writes the half-planes in the insertion's banded
     layout (Settings.Layout.kBanded inputs), so that fr_execute inserts from them without a copy."""
 
     def __init__(self, size_x: int, size_y: int, out_x: int = 0, out_y: int = 0, normalize: bool = True,
