@@ -148,6 +148,7 @@ static void set_table(frb::InsertParams &P, const fr_handle *h, const float *tab
     P.tableElems = frb::kKaiserTableElems;
     P.tableScale = float(frb::kKaiserTableElems - 1) / (s.blob_radius * s.blob_radius);
   }
+  std::copy(h->kaiser.begin(), h->kaiser.end(), P.kaiser);
 }
 
 int check_settings(const fr_settings *s)
@@ -181,7 +182,39 @@ bool is_host_pointer(const void *p)
 
 }// namespace
 
+// Interpolation at kKaiserDegree + 1 Chebyshev points of [0, 1] raised to 1.5, which crowds them
+// towards u = 0 -- the blob's edge, where the weight is 1 / I0(alpha) of its peak -- so that the
+// relative error there stays at FP32's; Newton's divided differences, expanded to powers of u.
+void frb::kaiser_polynomial(float alpha, float ks, float2 (&c)[kKaiserDegree + 1])
+{
+  constexpr int n = kKaiserDegree + 1;
+  double u[n], f[n], a[n] = {};
+  for (int k = 0; k < n; ++k) {
+    u[k] = std::pow(0.5 - 0.5 * std::cos(3.14159265358979323846 * (k + 0.5) / n), 1.5);
+    // I0(x) = sum over m of (x^2 / 4)^m / (m!)^2; 60 terms leave nothing for x <= 15
+    const double q = 0.25 * double(alpha) * double(alpha) * u[k];
+    double term = 1.0, sum = 1.0;
+    for (int m = 1; m < 60; ++m) sum += term *= q / (double(m) * m);
+    f[k] = sum;
+  }
+  for (int j = 1; j < n; ++j)
+    for (int k = n - 1; k >= j; --k) f[k] = (f[k] - f[k - 1]) / (u[k] - u[k - j]);
+  for (int j = n - 1; j >= 0; --j) {  // a(u) <- a(u) (u - u_j) + f_j
+    for (int k = n - 1; k > 0; --k) a[k] = a[k - 1] - u[j] * a[k];
+    a[0] = f[j] - u[j] * a[0];
+  }
+  for (int k = 0; k < n; ++k) c[k] = make_float2(float(a[k] * ks), float(a[k] * ks));
+}
+
 int frb::set_last_error(int code, const char *msg) { return fail(code, msg); }
+
+// The dynamic blob's polynomial for the handle's settings and constants.
+static void set_kaiser(fr_handle *h)
+{
+  float2 c[frb::kKaiserDegree + 1];
+  frb::kaiser_polynomial(h->constants.cBlobAlpha, h->constants.cOneOverBessiOrderAlpha * h->constants.cIw0, c);
+  std::copy(std::begin(c), std::end(c), h->kaiser.begin());
+}
 
 // Under FR_TUNING_CACHED / ON_EXECUTE, takes the launch parameters of an equal strategy's
 // tuning file (fr_init / fr_batch_init, after the dims or limits and settings are set).
@@ -415,6 +448,7 @@ int fr_init(fr_handle *h, const fr_dims *d, const fr_settings *s)
   g.cy = h->constants.cMaxVolumeIndexYZ / 2;
   g.cz = h->constants.cMaxVolumeIndexYZ / 2;
 
+  set_kaiser(h);
   frb::InsertConfig &cfg = h->cfg;
   cfg.fast = s->type == FR_TYPE_FAST;
   cfg.mode = s->interpolation == FR_INTERPOLATION_LOOKUP ? 0 : (s->alpha <= 15.f ? 1 : 3);
@@ -789,6 +823,7 @@ int fr_batch_init(fr_handle *h, const fr_batch_limits *lim, const fr_settings *s
   h->dims = fr_dims{};
   h->dims.table_elems = lim->table_elems;
   h->constants = make_constants(3, 3, s->interpolation == FR_INTERPOLATION_LOOKUP ? lim->table_elems : 0, *s);
+  set_kaiser(h);
   frb::InsertConfig &cfg = h->cfg;
   fill_config(cfg, *s);
   cfg.jobs = true;

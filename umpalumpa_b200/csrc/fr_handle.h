@@ -34,6 +34,7 @@ struct fr_handle {
   fr_dims dims{};
   fr_settings settings{};
   fr_constants constants{};
+  std::array<float2, frb::kKaiserDegree + 1> kaiser{};  // dynamic blob, alpha <= 15 (kaiser_polynomial)
   frb::BinGeom geom{};
   frb::InsertConfig cfg{};
   fr_launch_params launch{};

@@ -246,7 +246,7 @@ __device__ __forceinline__ bool voxel_blob(const InsertParams &P, const JobGeom 
   for (int k = 0; k < TAPS / 2; ++k) dxp[k] = make_float2(dx0 - float(2 * k), dx0 - float(2 * k + 1));
   const float2 cI2 = make_float2(c.cIDeltaSqrt, c.cIDeltaSqrt);
   const float2 kt2 = make_float2(P.tableScale, P.tableScale);
-  const float alpha2 = c.cBlobAlpha * c.cBlobAlpha, ks = c.cOneOverBessiOrderAlpha * c.cIw0;
+  const float2 negInvR2 = make_float2(-c.cOneOverBlobRadiusSqr, -c.cOneOverBlobRadiusSqr);
   const float2 half2 = make_float2(0.5f, 0.5f);
   float2 acc = make_float2(0.f, 0.f);
   float w = 0.f;
@@ -267,7 +267,7 @@ __device__ __forceinline__ bool voxel_blob(const InsertParams &P, const JobGeom 
         const float2 e = reinterpret_cast<const float2 *>(lut)[li];
         wb = fmaf(e.y, pos - float(li), e.x);
       } else if (MODE == kModeFastKaiser) {
-        wb = pos;  // the pair's weights, computed below with kaiser_value_fast2
+        wb = pos;  // the pair's weights, computed below with kaiser_poly2
       } else {
         wb = kaiser_value_f(sqrtf(d2), r, c.cBlobAlpha, c.cOneOverBessiOrderAlpha, P.order) * c.cIw0;
       }
@@ -288,7 +288,7 @@ __device__ __forceinline__ bool voxel_blob(const InsertParams &P, const JobGeom 
       // per tap: the table position (lookup), the blob weight (fast Kaiser) or d2
       const float2 pos = MODE == kModeLut            ? __ffma2_rn(d2, cI2, half2)
                          : MODE == kModeKaiserTable ? __fmul2_rn(d2, kt2)
-                         : MODE == kModeFastKaiser  ? kaiser_value_fast2(d2, alpha2, c.cOneOverBlobRadiusSqr, ks)
+                         : MODE == kModeFastKaiser  ? kaiser_poly2(d2, negInvR2, P.kaiser)
                                                     : d2;
       tap(row, ii, 2 * k, d2.x, pos.x);
       tap(row, ii, 2 * k + 1, d2.y, pos.y);

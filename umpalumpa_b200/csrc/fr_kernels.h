@@ -56,6 +56,9 @@ constexpr int kItemsPerGroup = 4;
 constexpr int kFastItemsPerGroup = 1;  // nearest pixel: an entry costs a tenth of a blob entry
 
 
+// Degree of the dynamic blob's polynomial (alpha <= 15).
+constexpr int kKaiserDegree = 12;
+
 struct InsertParams {
   const JobDesc *jobs;  // batched launches: the job table (the per-job fields below unused)
   void *volume;
@@ -71,6 +74,7 @@ struct InsertParams {
   const float *table;  // lookup: the blob table; dynamic: the Kaiser (value, slope) table
   int tableElems;      // entries (float2 entries for the Kaiser table)
   float tableScale;    // Kaiser table: nodes per unit of d^2, (N - 1) / r^2
+  float2 kaiser[kKaiserDegree + 1];  // dynamic, alpha <= 15: kaiser_polynomial, each coefficient twice
   int lutInSmem;
   int genericTaps;  // bounds-checked taps with a clamped table index: half-plane narrower or
                     // shorter than the blob window, or a blob table above kLutSmemMax entries
@@ -111,6 +115,9 @@ InsertFn pick_insert_batch_fp32(const InsertConfig &cfg);
 InsertFn pick_insert_batch_bf16(const InsertConfig &cfg);
 InsertFn pick_insert_batch_fp16(const InsertConfig &cfg);
 
+// Coefficients, constant first, of the polynomial in u = 1 - d2 / r^2 that interpolates
+// ks I0(alpha sqrt(u)), |alpha| <= 15.
+void kaiser_polynomial(float alpha, float ks, float2 (&c)[kKaiserDegree + 1]);
 // Dynamic interpolation's Kaiser (value, slope) table: kKaiserTableElems float2 entries.
 cudaError_t launch_kaiser_table(float *table, int order, float alpha, float radius, float iw0, cudaStream_t st);
 cudaError_t launch_blob_table(float *table, int64_t n, int order, float alpha, float radius,

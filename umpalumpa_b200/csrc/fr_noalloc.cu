@@ -250,6 +250,7 @@ extern "C" int fr_insert_noalloc(int device, void *stream, const fr_dims *d, con
                              : int(s->interpolation == FR_INTERPOLATION_LOOKUP ? d->table_elems : 0);
   P.tableScale = kaiserTable ? float(frb::kKaiserTableElems - 1) / (s->blob_radius * s->blob_radius) : 0.f;
   P.lutInSmem = frb::insert_lut_in_smem(cfg, P.tableElems);
+  frb::kaiser_polynomial(c.cBlobAlpha, c.cOneOverBessiOrderAlpha * c.cIw0, P.kaiser);
   P.genericTaps = int(d->fft_x) < cfg.taps || int(d->fft_y) < cfg.taps || P.tableElems > frb::kLutSmemMax;
   P.c = c;
   P.order = s->blob_order;
