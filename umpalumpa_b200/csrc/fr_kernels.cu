@@ -756,7 +756,7 @@ ItemSplit item_split(int itemCapacity, int brickGroups, const InsertConfig &cfg)
   return { itemCapacity, itemCapacity == kItemCapacity ? perGroup * brickGroups : 0, cfg.fast ? 32 : 2, cfg.kahan ? 8 : 0 };
 }
 
-int insert_max_groups(const InsertConfig &cfg) { return cfg.kahan ? 2 : 3; }
+int insert_max_groups(const InsertConfig &cfg) { return (cfg.kahan ? 2 : 3) + (cfg.fast ? 1 : 0); }
 
 int insert_groups(const InsertConfig &cfg)
 {
