@@ -6,12 +6,34 @@
 
 namespace frb {
 
+// A traverse space by 16-byte loads where the caller's array allows them (it starts on a 16-byte
+// boundary; a space is 7 x 16 bytes), else field by field.
+__device__ __forceinline__ fr_traverse_space load_space(const fr_traverse_space *p)
+{
+  if (reinterpret_cast<uintptr_t>(p) & 15) return *p;
+  fr_traverse_space s;
+  const float4 *q = reinterpret_cast<const float4 *>(p);
+  float4 *d = reinterpret_cast<float4 *>(&s);
+#pragma unroll
+  for (int k = 0; k < 7; ++k) d[k] = __ldg(q + k);
+  return s;
+}
+
+template<typename T> __device__ __forceinline__ T pick3(int k, T a, T b, T c) { return k == 0 ? a : (k == 1 ? b : c); }
+
 // Builds, for one space, the binning record (SpacePrep) and the insertion record (SpaceRec)
 // relative to the volume centre (cx, cy, cz).  A space whose projectionIndex is outside the
 // FFT payload is given direction -1, so it is never binned (never read); returns false then.
+// Bound by latency -- a call has few spaces per SM: the FP64 part takes two quotients, and no
+// array is indexed by the direction (13 -> 3.6 us for a thousand spaces).
 __device__ __forceinline__ bool prep_space(const fr_traverse_space &s, float halfWidth, float xMin,
   float radius, int cx, int cy, int cz, int nProj, SpacePrep &p, SpaceRec &r)
 {
+  const int dir = s.dir;
+  const int ua = dir == FR_DIR_YZ ? 1 : 0;
+  const int va = dir == FR_DIR_XY ? 1 : 2;
+  const int wa = dir == FR_DIR_XY ? 2 : (dir == FR_DIR_XZ ? 1 : 0);
+  const int open = 1 << 30;
   for (int k = 0; k < 3; ++k) {
     p.t0[k] = s.transformInv[0][k];
     p.t2[k] = s.transformInv[2][k];
@@ -19,154 +41,195 @@ __device__ __forceinline__ bool prep_space(const fr_traverse_space &s, float hal
   p.maxDist2 = s.maxDistanceSqr * 1.00001f + 1e-2f;
   p.halfWidth = halfWidth;
   p.xMin = xMin;
-  const int open = 1 << 30;
-  int lo[3] = { s.minX, s.minY, s.minZ }, hi[3] = { s.maxX, s.maxY, s.maxZ };
-  const int dir = s.dir;
-  const int ua = dir == FR_DIR_YZ ? 1 : 0;
-  const int va = dir == FR_DIR_XY ? 1 : 2;
-  const int wa = dir == FR_DIR_XY ? 2 : (dir == FR_DIR_XZ ? 1 : 0);
-  const int far = 1 << 24;  // floats hold every integer up to here
-  r.lo0 = float(min(max(lo[ua], -far), far));
-  r.hi0 = float(min(max(hi[ua], -far), far));
-  r.lo1 = float(min(max(lo[va], -far), far));
-  r.hi1 = float(min(max(hi[va], -far), far));
-  lo[wa] = -open;
-  hi[wa] = open;
-  for (int k = 0; k < 3; ++k) {
-    p.lo[k] = lo[k];
-    p.hi[k] = hi[k];
-  }
-  p.dir = dir;
+  p.lo[0] = wa == 0 ? -open : s.minX;
+  p.lo[1] = wa == 1 ? -open : s.minY;
+  p.lo[2] = wa == 2 ? -open : s.minZ;
+  p.hi[0] = wa == 0 ? open : s.maxX;
+  p.hi[1] = wa == 1 ? open : s.maxY;
+  p.hi[2] = wa == 2 ? open : s.maxZ;
   const bool bad = s.projectionIndex < 0 || s.projectionIndex >= nProj;
-  if (bad) p.dir = -1;  // matches no direction segment
+  p.dir = bad ? -1 : dir;  // -1 matches no direction segment
 
+  const int far = 1 << 24;  // floats hold every integer up to here
+  r.lo0 = float(min(max(pick3(ua, s.minX, s.minY, s.minZ), -far), far));
+  r.hi0 = float(min(max(pick3(ua, s.maxX, s.maxY, s.maxZ), -far), far));
+  r.lo1 = float(min(max(pick3(va, s.minX, s.minY, s.minZ), -far), far));
+  r.hi1 = float(min(max(pick3(va, s.maxX, s.maxY, s.maxZ), -far), far));
   for (int k = 0; k < 9; ++k) r.T[k] = s.transformInv[k / 3][k % 3];
   r.maxDist2 = s.maxDistanceSqr;
   r.weight = s.weight;
   r.proj = s.projectionIndex;
-  const double c[3] = { double(cx), double(cy), double(cz) };
-  const double nrm[3] = { s.transformInv[2][0], s.transformInv[2][1], s.transformInv[2][2] };
-  const double nw = nrm[wa];
+  const double cu = pick3(ua, cx, cy, cz), cv = pick3(va, cx, cy, cz), cw = pick3(wa, cx, cy, cz);
+  const float (&t2)[3] = s.transformInv[2];
+  const double nu = pick3(ua, t2[0], t2[1], t2[2]), nv = pick3(va, t2[0], t2[1], t2[2]), nw = pick3(wa, t2[0], t2[1], t2[2]);
+  r.w0 = 0.f;  // degenerate normal: visit the whole column, the voxel checks decide
+  r.wu = 0.f;
+  r.wv = 0.f;
+  r.hw = 1e9f;
   if (fabs(nw) > 1e-6) {
-    r.w0 = float(c[wa] + (nrm[ua] * c[ua] + nrm[va] * c[va]) / nw);
-    r.wu = float(-nrm[ua] / nw);
-    r.wv = float(-nrm[va] / nw);
-    r.hw = float(double(radius) / fabs(nw) + 2e-3);
-  } else {  // degenerate normal: visit the whole column, the voxel checks decide
-    r.w0 = 0.f;
-    r.wu = 0.f;
-    r.wv = 0.f;
-    r.hw = 1e9f;
+    const double inv = 1.0 / nw;
+    r.w0 = float(cw + (nu * cu + nv * cv) * inv);
+    r.wu = float(-nu * inv);
+    r.wv = float(-nv * inv);
+    r.hw = float(double(radius) * fabs(inv) + 2e-3);
   }
   // half-space x' >= -r, with a margin of 0.01 in x' (far above the float error of h at the
   // largest volume, 1.5e-3 in x')
-  const double t0[3] = { s.transformInv[0][0], s.transformInv[0][1], s.transformInv[0][2] };
-  const double tw = t0[wa];
+  const float (&t0)[3] = s.transformInv[0];
+  const double tu = pick3(ua, t0[0], t0[1], t0[2]), tv = pick3(va, t0[0], t0[1], t0[2]), tw = pick3(wa, t0[0], t0[1], t0[2]);
   r.h0 = -1e30f;
   r.hu = 0.f;
   r.hv = 0.f;
   if (fabs(tw) > 1e-3) {
-    r.h0 = float(c[wa] + (t0[ua] * c[ua] + t0[va] * c[va] - double(radius) - 0.01) / tw);
-    r.hu = float(-t0[ua] / tw);
-    r.hv = float(-t0[va] / tw);
+    const double inv = 1.0 / tw;
+    r.h0 = float(cw + (tu * cu + tv * cv - double(radius) - 0.01) * inv);
+    r.hu = float(-tu * inv);
+    r.hv = float(-tv * inv);
     if (tw < 0) r.hw = -r.hw;
   }
   r.sphere = s.maxDistanceSqr;
-  const float *un = s.unitNormal, *bo = s.bottomOrigin;
-  r.nu = un[ua];
-  r.nv = un[va];
-  r.nw = un[wa];
-  r.bu = bo[ua];
-  r.bv = bo[va];
-  r.bw = bo[wa];
+  r.nu = pick3(ua, s.unitNormal[0], s.unitNormal[1], s.unitNormal[2]);
+  r.nv = pick3(va, s.unitNormal[0], s.unitNormal[1], s.unitNormal[2]);
+  r.nw = pick3(wa, s.unitNormal[0], s.unitNormal[1], s.unitNormal[2]);
+  r.bu = pick3(ua, s.bottomOrigin[0], s.bottomOrigin[1], s.bottomOrigin[2]);
+  r.bv = pick3(va, s.bottomOrigin[0], s.bottomOrigin[1], s.bottomOrigin[2]);
+  r.bw = pick3(wa, s.bottomOrigin[0], s.bottomOrigin[1], s.bottomOrigin[2]);
   r.pad[0] = r.pad[1] = 0;
   return !bad;
 }
 
-// Conservative test: can any voxel of the brick [b0, b1] (inclusive voxel coordinates)
-// receive a contribution from this space?  Centre (cx, cy, cz) is the reference's integer
-// volume centre.
-__device__ __forceinline__ bool brick_hit(const SpacePrep &p, const int b0[3], const int b1[3],
-  const float a[3], const float e[3])
+// Stores a record of 16-byte words.
+template<typename R> __device__ __forceinline__ void store_record(R *dst, const R &r)
 {
-  for (int k = 0; k < 3; ++k)
-    if (b1[k] < p.lo[k] || b0[k] > p.hi[k]) return false;
-  float zlo = 0.f, zhi = 0.f, xhi = 0.f, d2 = 0.f;
-  for (int k = 0; k < 3; ++k) {
-    float u = p.t2[k] * a[k], v = p.t2[k] * e[k];
-    zlo += fminf(u, v);
-    zhi += fmaxf(u, v);
-    xhi += fmaxf(p.t0[k] * a[k], p.t0[k] * e[k]);
-    float c = fminf(fmaxf(0.f, a[k]), e[k]);
-    d2 += c * c;
-  }
-  return zlo <= p.halfWidth && zhi >= -p.halfWidth && xhi >= p.xMin && d2 <= p.maxDist2;
+  static_assert(sizeof(R) % 16 == 0, "whole 16-byte words");
+  const float4 *s = reinterpret_cast<const float4 *>(&r);
+  float4 *d = reinterpret_cast<float4 *>(dst);
+#pragma unroll
+  for (int k = 0; k < int(sizeof(R) / 16); ++k) d[k] = s[k];
 }
 
-__device__ __forceinline__ void brick_box(const BinGeom &g, int b, int b0[3], int b1[3], float a[3],
-  float e[3])
+// One binning record through four 16-byte read-only loads.
+__device__ __forceinline__ SpacePrep load_prep(const SpacePrep *p)
 {
-  int bx = b % g.nbx, by = (b / g.nbx) % g.nby, bz = b / (g.nbx * g.nby);
-  int v[3] = { g.vx, g.vy, g.vz };
-  int c[3] = { g.cx, g.cy, g.cz };
-  int o[3] = { bx * kBrick, by * kBrick, bz * kBrick };
-  for (int k = 0; k < 3; ++k) {
-    b0[k] = o[k];
-    b1[k] = min(o[k] + kBrick, v[k]) - 1;
-    a[k] = float(b0[k] - c[k]);
-    e[k] = float(b1[k] - c[k]);
-  }
+  const float4 *q = reinterpret_cast<const float4 *>(p);
+  SpacePrep r;
+  float4 *d = reinterpret_cast<float4 *>(&r);
+  d[0] = __ldg(q);
+  d[1] = __ldg(q + 1);
+  d[2] = __ldg(q + 2);
+  d[3] = __ldg(q + 3);
+  return r;
 }
 
-// Union box of the bricks a binning CTA owns (bricks first .. first + count - 1): every space
-// that can touch one of them touches the union, so brick_hit on the union is a conservative
-// pre-test (the AABB overlap, the slab range, the half-space maximum and the distance of the
-// nearest point all widen with the box).
-__device__ __forceinline__ void union_box(const BinGeom &g, int first, int count, int u0[3], int u1[3], float ua[3],
-  float ue[3])
+// The (brick, direction) lists of up to kRowBricks bricks in a row along x (row `row` = y + nby z
+// of the brick grid, bricks bx0 ...; `brickBase` is added to the brick indices, `spaceBase` to the
+// listed space indices) by one 256-thread CTA.  A tile of 256 spaces at a time: every thread tests its
+// space against all bricks of the row -- the y and z parts of the tests are shared by the row --
+// and the hits go to shared memory as one bit mask per brick and warp; then FILL = false counts
+// them per (brick, direction), FILL = true has each warp write the hits of its bricks, in
+// ascending space order, into the bricks' three direction segments.  The next tile's records are
+// loaded during the tests; the masks are double-buffered, so a tile takes one barrier.
+//
+// The tests are conservative: can any voxel of the brick [b0, b1] (inclusive voxel coordinates,
+// relative to the reference's integer volume centre [a, e]) receive a contribution from the space?
+// The traversal box, the slab's range over the box, the half-space's maximum and the distance of
+// the box's nearest point decide.
+//
+// Bound by instruction issue (about 20 a space and brick).  A warp per brick testing the spaces
+// that hit the union of its CTA's eight bricks, compacted with three barriers a tile, took
+// 690 us per pass for 20,000 spaces at box 256 (now 180 counting, 325 filling) and 21 and 26 us for 1,013 at box 64 (now 5 and 9).
+constexpr int kRowBricks = 32;
+
+struct BinRow {
+  BinGeom g;
+  int row, bx0, n;            // n spaces from prep
+  int brickBase, spaceBase, job;
+  const SpacePrep *prep;
+};
+
+template<bool FILL>
+__device__ __forceinline__ void bin_row(const BinRow &R, int *__restrict__ counts, const int *__restrict__ offsets,
+  int *__restrict__ list, const BinBuffers &buf)
 {
-  for (int k = 0; k < 3; ++k) {
-    u0[k] = 1 << 30;
-    u1[k] = -(1 << 30);
-  }
-  for (int w = 0; w < count; ++w) {
-    int b0[3], b1[3];
-    float a[3], e[3];
-    brick_box(g, first + w, b0, b1, a, e);
-    for (int k = 0; k < 3; ++k) {
-      u0[k] = min(u0[k], b0[k]);
-      u1[k] = max(u1[k], b1[k]);
+  __shared__ unsigned hits[2][kRowBricks][8];
+  __shared__ unsigned dirs[2][8][3];
+  const BinGeom &g = R.g;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int nb = min(kRowBricks, g.nbx - R.bx0);
+  const int by = R.row % g.nby, bz = R.row / g.nby;
+  const int y0 = by * kBrick, z0 = bz * kBrick;
+  const int y1 = min(y0 + kBrick, g.vy) - 1, z1 = min(z0 + kBrick, g.vz) - 1;
+  const float ya = float(y0 - g.cy), ye = float(y1 - g.cy), za = float(z0 - g.cz), ze = float(z1 - g.cz);
+  const float yc = fminf(fmaxf(0.f, ya), ye), zc = fminf(fmaxf(0.f, za), ze);
+  const float yz2 = yc * yc + zc * zc;
+  const int first = R.brickBase + (bz * g.nby + by) * g.nbx + R.bx0;  // the row's first brick
+  int count = 0;          // FILL = false: thread 3 b + d counts (brick b, direction d)
+  int at[4][3] = {};      // FILL = true: next list positions of bricks warp + 8 i
+  if (FILL)
+    for (int i = 0; i < 4; ++i)
+      for (int d = 0; d < 3; ++d)
+        if (warp + 8 * i < nb) at[i][d] = offsets[3 * (first + warp + 8 * i) + d];
+  SpacePrep next{};
+  if (tid < R.n) next = load_prep(R.prep + tid);
+  for (int base = 0, t = 0; base < R.n; base += 256, t ^= 1) {
+    const SpacePrep p = next;
+    const bool live = base + tid < R.n;
+    if (base + 256 + tid < R.n) next = load_prep(R.prep + base + 256 + tid);
+    const bool row = live && y1 >= p.lo[1] && y0 <= p.hi[1] && z1 >= p.lo[2] && z0 <= p.hi[2];
+    const float zl = fminf(p.t2[1] * ya, p.t2[1] * ye) + fminf(p.t2[2] * za, p.t2[2] * ze) - p.halfWidth;
+    const float zh = fmaxf(p.t2[1] * ya, p.t2[1] * ye) + fmaxf(p.t2[2] * za, p.t2[2] * ze) + p.halfWidth;
+    const float xh = fmaxf(p.t0[1] * ya, p.t0[1] * ye) + fmaxf(p.t0[2] * za, p.t0[2] * ze) - p.xMin;
+    const float left = p.maxDist2 - yz2;
+    for (int d = 0; d < 3; ++d) {
+      const unsigned m = __ballot_sync(0xffffffffu, live && p.dir == d);
+      if (lane == 0) dirs[t][warp][d] = m;
+    }
+    for (int b = 0; b < nb; ++b) {
+      const int x0 = (R.bx0 + b) * kBrick, x1 = min(x0 + kBrick, g.vx) - 1;
+      const float xa = float(x0 - g.cx), xe = float(x1 - g.cx);
+      const float xc = fminf(fmaxf(0.f, xa), xe);
+      const float u = p.t2[0] * xa, v = p.t2[0] * xe;
+      const bool hit = row && x1 >= p.lo[0] && x0 <= p.hi[0] && zl + fminf(u, v) <= 0.f && zh + fmaxf(u, v) >= 0.f
+                       && xh + fmaxf(p.t0[0] * xa, p.t0[0] * xe) >= 0.f && xc * xc <= left;
+      const unsigned m = __ballot_sync(0xffffffffu, hit);
+      if (lane == 0) hits[t][b][warp] = m;
+    }
+    __syncthreads();
+    if (!FILL) {
+      if (tid < 3 * nb) {
+        const int b = tid / 3, d = tid - 3 * b;
+#pragma unroll
+        for (int w = 0; w < 8; ++w) count += __popc(hits[t][b][w] & dirs[t][w][d]);
+      }
+    } else {
+      const unsigned before = (1u << lane) - 1u;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        if (warp + 8 * i >= nb) break;
+        for (int w = 0; w < 8; ++w) {
+          const unsigned m = hits[t][warp + 8 * i][w];
+          if (m == 0) continue;
+#pragma unroll
+          for (int d = 0; d < 3; ++d) {
+            const unsigned md = m & dirs[t][w][d];
+            if (md >> lane & 1u) list[at[i][d] + __popc(md & before)] = R.spaceBase + base + 32 * w + lane;
+            at[i][d] += __popc(md);
+          }
+        }
+      }
     }
   }
-  const int c[3] = { g.cx, g.cy, g.cz };
-  for (int k = 0; k < 3; ++k) {
-    ua[k] = float(u0[k] - c[k]);
-    ue[k] = float(u1[k] - c[k]);
+  if (!FILL) {
+    if (tid < 3 * nb) counts[3 * first + tid] = count;
+    return;
   }
-}
-
-// Compacts, in ascending order, the tile entries [0, m) that hit the union box into idx[0, *n)
-// (every thread of the 256-thread CTA calls it; ends with a barrier).
-__device__ __forceinline__ void compact_tile_hits(const SpacePrep *tile, int m, const int u0[3], const int u1[3],
-  const float ua[3], const float ue[3], int *idx, int *n, int *warpBase)
-{
-  const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
-  const bool h = t < m && brick_hit(tile[t], u0, u1, ua, ue);
-  const unsigned mask = __ballot_sync(0xffffffffu, h);
-  if (lane == 0) warpBase[warp] = __popc(mask);
-  __syncthreads();
-  if (t == 0) {
-    int run = 0;
-    for (int w = 0; w < 8; ++w) {
-      const int c = warpBase[w];
-      warpBase[w] = run;
-      run += c;
-    }
-    *n = run;
+  // the bricks' work items: at most `cap` list entries each, from the plan's first item on
+  const int cap = *buf.itemCap;
+  for (int b = warp; b < nb; b += 8) {
+    const int brick = first + b, beg = offsets[3 * brick], end = offsets[3 * brick + 3], item = buf.itemStart[brick];
+    for (int q = lane; beg + q * cap < end; q += 32)
+      buf.items[item + q] = { brick, beg + q * cap, min(end, beg + (q + 1) * cap), R.job };
   }
-  __syncthreads();
-  if (h) idx[warpBase[warp] + __popc(mask & ((1u << lane) - 1u))] = t;
-  __syncthreads();
 }
 
 }// namespace frb

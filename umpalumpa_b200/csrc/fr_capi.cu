@@ -306,9 +306,13 @@ int fr_create(int device, void *stream, fr_handle **out)
     e = cudaGetDeviceProperties(&prop, device);
     if (e == cudaSuccess) h->device_name = prop.name;
   }
-  if (e == cudaSuccess) e = cudaHostAlloc(reinterpret_cast<void **>(&h->host_status), 64, cudaHostAllocDefault);
-  if (e == cudaSuccess)
-    e = cudaHostAlloc(reinterpret_cast<void **>(&h->host_stats), 4 * sizeof(unsigned long long), cudaHostAllocDefault);
+  if (e == cudaSuccess) e = cudaHostAlloc(reinterpret_cast<void **>(&h->host_misc), frb::kMiscBytes, cudaHostAllocDefault);
+  if (e == cudaSuccess) {
+    std::memset(h->host_misc, 0, frb::kMiscBytes);
+    h->host_status = h->host_misc + frb::kMiscStatus;
+    h->host_stats = reinterpret_cast<unsigned long long *>(h->host_misc + frb::kMiscStats);
+    frb::prefer_shared_carveout();
+  }
   if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&h->copy_stream, cudaStreamNonBlocking);
   if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&h->band_stream, cudaStreamNonBlocking);
   if (e == cudaSuccess) e = cudaEventCreateWithFlags(&h->band_fork, cudaEventDisableTiming);
@@ -318,8 +322,7 @@ int fr_create(int device, void *stream, fr_handle **out)
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&h->slots[k].free, cudaEventDisableTiming);
   }
   if (e != cudaSuccess) {
-    if (h->host_status) cudaFreeHost(h->host_status);
-    if (h->host_stats) cudaFreeHost(h->host_stats);
+    if (h->host_misc) cudaFreeHost(h->host_misc);
     for (auto &sl : h->slots) {
       if (sl.ready) cudaEventDestroy(sl.ready);
       if (sl.free) cudaEventDestroy(sl.free);
@@ -388,8 +391,7 @@ int fr_destroy(fr_handle *h)
   if (h->band_join) cudaEventDestroy(h->band_join);
   if (h->band_stream) cudaStreamDestroy(h->band_stream);
   if (h->copy_stream) cudaStreamDestroy(h->copy_stream);
-  if (h->host_status) cudaFreeHost(h->host_status);
-  if (h->host_stats) cudaFreeHost(h->host_stats);
+  if (h->host_misc) cudaFreeHost(h->host_misc);
   delete h;
   return FR_OK;
 }
@@ -510,7 +512,6 @@ int fr_init(fr_handle *h, const fr_dims *d, const fr_settings *s)
   const size_t oOrder = take(size_t(g.n_bricks) * sizeof(int));
   const size_t oItems = take(size_t(itemsCap) * frb::kWorkItemBytes);
   const size_t oMisc = take(64);
-  const size_t oStats = take(4 * sizeof(unsigned long long));
   const size_t oKaiser = take(cfg.mode == 3 && !cfg.fast ? size_t(frb::kKaiserTableElems) * sizeof(float2) : 0);
   FR_CUDA(cudaMalloc(&h->scratch, off));
   h->scratch_bytes = off;
@@ -524,15 +525,11 @@ int fr_init(fr_handle *h, const fr_dims *d, const fr_settings *s)
   bb.order = reinterpret_cast<const int *>(base + oOrder);
   bb.items = reinterpret_cast<frb::WorkItem *>(base + oItems);
   int *misc = reinterpret_cast<int *>(base + oMisc);
-  bb.nItems = misc;
-  bb.status = misc + 1;
-  h->work_counter = misc + 2;
-  bb.stats = reinterpret_cast<unsigned long long *>(base + oStats);
+  frb::set_misc(bb, misc);
   bb.listCap = listCap;
   bb.itemsCap = itemsCap;
   FR_CUDA(cudaMemcpyAsync(base + oOrder, order.data(), order.size() * sizeof(int), cudaMemcpyHostToDevice, h->stream));
   FR_CUDA(cudaMemsetAsync(misc, 0, 64, h->stream));
-  FR_CUDA(cudaMemsetAsync(bb.stats, 0, 4 * sizeof(unsigned long long), h->stream));
   h->kaiser_table = nullptr;
   if (cfg.mode == 3 && !cfg.fast) {
     h->kaiser_table = reinterpret_cast<float *>(base + oKaiser);
@@ -736,7 +733,7 @@ int fr_execute(fr_handle *h, const void *fft, const float *scales, uint64_t nPro
   P.offsets = h->bb.offsets;
   P.items = h->bb.items;
   P.nItems = h->bb.nItems;
-  P.workCounter = h->work_counter;
+  P.workCounter = h->bb.workCounter;
   set_table(P, h, table, h->dims.table_elems);
   P.lutInSmem = frb::insert_lut_in_smem(h->cfg, P.tableElems);
   P.genericTaps = int(h->dims.fft_x) < h->cfg.taps || int(h->dims.fft_y) < h->cfg.taps || P.tableElems > frb::kLutSmemMax;
@@ -757,14 +754,12 @@ int fr_execute(fr_handle *h, const void *fft, const float *scales, uint64_t nPro
   P.cz = h->geom.cz;
 
   uint64_t launches = 0;
-  FR_CUDA(cudaMemsetAsync(h->bb.stats, 0, 4 * sizeof(unsigned long long), h->stream));
   for (uint64_t s0 = 0; s0 < nSpaces; s0 += uint64_t(h->chunk_cap)) {
     const int n = int(std::min<uint64_t>(uint64_t(h->chunk_cap), nSpaces - s0));
     int e0 = -1, e1 = -1, e2 = -1;
     if (h->profiling) FR_CUDA(cudaEventRecord(next_event(h, e0), h->stream));
     FR_CUDA(frb::launch_binning(h->geom, spaces + s0, n, int(nProj), h->cfg.fast, s.blob_radius, h->bb,
-      handle_split(h), h->stream));
-    FR_CUDA(cudaMemsetAsync(h->work_counter, 0, sizeof(int), h->stream));
+      handle_split(h), s0 == 0, h->stream));
     if (bandCopy && s0 == 0) FR_CUDA(cudaStreamWaitEvent(h->stream, h->band_join, 0));
     if (h->profiling) FR_CUDA(cudaEventRecord(next_event(h, e1), h->stream));
     FR_CUDA(frb::launch_insert(P, h->cfg, h->grid, h->stream));
@@ -781,8 +776,7 @@ int fr_execute(fr_handle *h, const void *fft, const float *scales, uint64_t nPro
     slot->used = true;
   }
   h->launches_pending += launches + (bandCopy ? 1 : 0);
-  FR_CUDA(cudaMemcpyAsync(h->host_stats, h->bb.stats, 4 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, h->stream));
-  FR_CUDA(cudaMemcpyAsync(h->host_status, h->bb.status, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
+  FR_CUDA(cudaMemcpyAsync(h->host_misc, h->bb.nItems, frb::kMiscBytes, cudaMemcpyDeviceToHost, h->stream));
   return FR_OK;
 }
 
@@ -866,7 +860,6 @@ int fr_batch_init(fr_handle *h, const fr_batch_limits *lim, const fr_settings *s
   const size_t oItems = take(size_t(itemsCap) * frb::kWorkItemBytes);
   const size_t oJobs = take(size_t(lim->max_jobs) * sizeof(frb::JobDesc));
   const size_t oMisc = take(64);
-  const size_t oStats = take(4 * sizeof(unsigned long long));
   const size_t oKaiser = take(cfg.mode == 3 && !cfg.fast ? size_t(frb::kKaiserTableElems) * sizeof(float2) : 0);
   FR_CUDA(cudaMalloc(&h->scratch, off));
   h->scratch_bytes = off;
@@ -880,10 +873,7 @@ int fr_batch_init(fr_handle *h, const fr_batch_limits *lim, const fr_settings *s
   bb.order = reinterpret_cast<const int *>(base + oOrder);
   bb.items = reinterpret_cast<frb::WorkItem *>(base + oItems);
   int *misc = reinterpret_cast<int *>(base + oMisc);
-  bb.nItems = misc;
-  bb.status = misc + 1;
-  h->work_counter = misc + 2;
-  bb.stats = reinterpret_cast<unsigned long long *>(base + oStats);
+  frb::set_misc(bb, misc);
   bb.listCap = listCap;
   bb.itemsCap = itemsCap;
   h->d_jobs = reinterpret_cast<frb::JobDesc *>(base + oJobs);
@@ -898,7 +888,6 @@ int fr_batch_init(fr_handle *h, const fr_batch_limits *lim, const fr_settings *s
   h->h_order = h->h_order_set[0];
   h->upload_done = h->upload_set_done[0];
   FR_CUDA(cudaMemsetAsync(misc, 0, 64, h->stream));
-  FR_CUDA(cudaMemsetAsync(bb.stats, 0, 4 * sizeof(unsigned long long), h->stream));
   h->kaiser_table = nullptr;
   if (cfg.mode == 3 && !cfg.fast) {
     h->kaiser_table = reinterpret_cast<float *>(base + oKaiser);
@@ -925,10 +914,8 @@ static int enqueue_batch(fr_handle *h, int nJobs, int totalSpaces, int totalBric
   FR_CUDA(cudaStreamWaitEvent(h->band_stream, h->band_fork, 0));
   FR_CUDA(frb::launch_batch_band(h->d_jobs, nJobs, bandUnits, s.storage == FR_STORAGE_FP32 ? 8 : 4, h->band_stream));
   FR_CUDA(cudaEventRecord(h->band_join, h->band_stream));
-  FR_CUDA(cudaMemsetAsync(h->bb.stats, 0, 4 * sizeof(unsigned long long), h->stream));
   FR_CUDA(frb::launch_batch_binning(h->d_jobs, nJobs, totalSpaces, totalBricks, totalGroups, h->cfg.fast,
     s.blob_radius, h->bb, handle_split(h), h->stream));
-  FR_CUDA(cudaMemsetAsync(h->work_counter, 0, sizeof(int), h->stream));
   FR_CUDA(cudaStreamWaitEvent(h->stream, h->band_join, 0));
   frb::InsertParams P{};
   P.jobs = h->d_jobs;
@@ -937,14 +924,13 @@ static int enqueue_batch(fr_handle *h, int nJobs, int totalSpaces, int totalBric
   P.offsets = h->bb.offsets;
   P.items = h->bb.items;
   P.nItems = h->bb.nItems;
-  P.workCounter = h->work_counter;
+  P.workCounter = h->bb.workCounter;
   set_table(P, h, table, h->blim.table_elems);
   P.lutInSmem = frb::insert_lut_in_smem(h->cfg, P.tableElems);
   P.c = h->constants;
   P.order = s.blob_order;
   FR_CUDA(frb::launch_insert(P, h->cfg, h->grid, h->stream));
-  FR_CUDA(cudaMemcpyAsync(h->host_stats, h->bb.stats, 4 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, h->stream));
-  FR_CUDA(cudaMemcpyAsync(h->host_status, h->bb.status, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
+  FR_CUDA(cudaMemcpyAsync(h->host_misc, h->bb.nItems, frb::kMiscBytes, cudaMemcpyDeviceToHost, h->stream));
   return FR_OK;
 }
 
@@ -1019,7 +1005,7 @@ int fr_batch_execute(fr_handle *h, const fr_job *jobs, uint64_t nJobs, const flo
     }
     spaceBase += int64_t(J.n_spaces);
     brickBase += D.nBricks;
-    groupBase += (D.nBricks + 7) / 8;
+    groupBase += frb::bin_groups(D.nbx, D.nby, D.nbz);
     if (bandUnits > int64_t(INT32_MAX)) return fail(FR_E_UNSUPPORTED, "too many projection rows in one batch");
   }
   if (spaceBase > int64_t(h->blim.max_spaces) || brickBase > int64_t(h->blim.max_bricks))

@@ -91,7 +91,7 @@ struct JobDesc {
   int vy, vz, nbx, nby;
   int nbz, cx, cy, cz;
   int genericTaps, spaceBase, nSpaces, brickBase;
-  int nBricks, groupBase;              // bricks; first 8-brick binning group of the job
+  int nBricks, groupBase;              // bricks; first binning CTA of the job (bin_groups)
   const fr_traverse_space *spaces;     // the job's traverse spaces (device memory)
   const void *src;                     // the caller's row-major half-planes (fft: their bands)
   int bandStride;                      // elements per 4-row band of fft

@@ -43,9 +43,9 @@ struct fr_handle {
   void *scratch = nullptr;
   size_t scratch_bytes = 0;
   frb::BinBuffers bb{};
-  int *work_counter = nullptr;
-  int *host_status = nullptr;                 // pinned: status + padding
-  unsigned long long *host_stats = nullptr;   // pinned: 4 counters
+  int *host_misc = nullptr;                   // pinned mirror of the scratch's small words (set_misc)
+  int *host_status = nullptr;                 // in it: the status
+  unsigned long long *host_stats = nullptr;   // in it: the call's counters
   StageSlot slots[2];
   int next_slot = 0;
   // Banded copy of the projections (FR_LAYOUT_AUTO and batches): written on band_stream while

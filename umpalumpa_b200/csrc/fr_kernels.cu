@@ -249,92 +249,26 @@ __global__ void space_prep_kernel(const fr_traverse_space *__restrict__ spaces, 
   if (i >= n) return;
   SpacePrep p;
   SpaceRec r;
-  if (!prep_space(spaces[i], halfWidth, xMin, radius, cx, cy, cz, nProj, p, r)) atomicCAS(status, 0, FR_E_INVALID);
-  out[i] = p;
-  rec[i] = r;
+  if (!prep_space(load_space(spaces + i), halfWidth, xMin, radius, cx, cy, cz, nProj, p, r)) atomicCAS(status, 0, FR_E_INVALID);
+  store_record(out + i, p);
+  store_record(rec + i, r);
 }
 
-// One warp per brick, 8 bricks per CTA; the CTA stages 256 space records at a time in
-// shared memory, keeps those that hit the union box of its bricks (in ascending order) and
-// only those are tested per brick.  FILL = false counts hits per (brick, direction); FILL =
-// true writes the hit space indices in ascending order into the brick's three direction
-// segments.
-// The band copy, the binning and the insertion all ask for the largest shared-memory carve-out,
-// so that an SM running copy CTAs (which need no shared memory) can take binning CTAs beside
-// them instead of waiting for the copy to end.
-template<typename K> static void prefer_max_shared(K *kernel)
-{
-  if (cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared)
-      != cudaSuccess)
-    cudaGetLastError();  // a hint only
-}
-
-// One binning record through four 16-byte read-only loads.  The binning kernels fetch the next
-// 256 records into registers while they test the staged ones, so the load latency hides behind
-// the tests (without it the stages waited on their loads, and a copy kernel running beside the
-// binning, as the band copy does, doubled the binning time).
-__device__ __forceinline__ SpacePrep load_prep(const SpacePrep *p)
-{
-  const float4 *q = reinterpret_cast<const float4 *>(p);
-  SpacePrep r;
-  float4 *d = reinterpret_cast<float4 *>(&r);
-  d[0] = __ldg(q);
-  d[1] = __ldg(q + 1);
-  d[2] = __ldg(q + 2);
-  d[3] = __ldg(q + 3);
-  return r;
-}
-
+// The lists of one row of bricks (bin_row).  FILL does nothing once the status is set: the plan
+// then publishes no items, and the lists would not be read.
 template<bool FILL>
-__global__ void __launch_bounds__(256) bin_kernel(BinGeom g, const SpacePrep *__restrict__ prep,
-  int n, int *__restrict__ counts, const int *__restrict__ offsets, int *__restrict__ list,
-  const int *__restrict__ status)
+__global__ void __launch_bounds__(256) bin_kernel(BinGeom g, const SpacePrep *__restrict__ prep, int n, BinBuffers b)
 {
-  __shared__ SpacePrep tile[256];
-  __shared__ int hitIdx[256];
-  __shared__ int hitN, warpBase[8];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int b = blockIdx.x * 8 + warp;
-  const bool active = b < g.n_bricks;
-  if (FILL && *status != 0) return;
-  int b0[3] = {}, b1[3] = {};
-  float a[3] = {}, e[3] = {};
-  if (active) brick_box(g, b, b0, b1, a, e);
-  int u0[3], u1[3];
-  float ua[3], ue[3];
-  union_box(g, blockIdx.x * 8, min(8, g.n_bricks - int(blockIdx.x) * 8), u0, u1, ua, ue);
-  int cnt[3] = { 0, 0, 0 };
-  if (FILL && active)
-    for (int d = 0; d < 3; ++d) cnt[d] = offsets[3 * b + d];
-  SpacePrep next;
-  if (int(threadIdx.x) < n) next = load_prep(prep + threadIdx.x);
-  for (int base = 0; base < n; base += 256) {
-    __syncthreads();
-    if (base + int(threadIdx.x) < n) tile[threadIdx.x] = next;
-    __syncthreads();
-    if (base + 256 + int(threadIdx.x) < n) next = load_prep(prep + base + 256 + threadIdx.x);
-    const int m = min(256, n - base);
-    compact_tile_hits(tile, m, u0, u1, ua, ue, hitIdx, &hitN, warpBase);
-    if (!active) continue;
-    const int hn = hitN;
-    for (int r = 0; r < hn; r += 32) {
-      const int jj = r + lane;
-      bool hit = false;
-      int dir = 0, j = 0;
-      if (jj < hn) {
-        j = hitIdx[jj];
-        hit = brick_hit(tile[j], b0, b1, a, e);
-        dir = tile[j].dir;
-      }
-      for (int d = 0; d < 3; ++d) {
-        unsigned mask = __ballot_sync(0xffffffffu, hit && dir == d);
-        if (FILL && hit && dir == d) list[cnt[d] + __popc(mask & ((1u << lane) - 1u))] = base + j;
-        cnt[d] += __popc(mask);
-      }
-    }
-  }
-  if (!FILL && active && lane == 0)
-    for (int d = 0; d < 3; ++d) counts[3 * b + d] = cnt[d];
+  if (FILL && *b.status != 0) return;
+  BinRow R;
+  R.g = g;
+  const int rows = g.nby * g.nbz;
+  R.row = blockIdx.x % rows;
+  R.bx0 = blockIdx.x / rows * kRowBricks;
+  R.n = n;
+  R.brickBase = R.spaceBase = R.job = 0;
+  R.prep = prep;
+  bin_row<FILL>(R, b.counts, b.offsets, b.list, b);
 }
 
 // ---- batched binning: the spaces and bricks of several jobs, indexed batch-wide ----------
@@ -361,184 +295,127 @@ __global__ void batch_prep_kernel(const JobDesc *__restrict__ jobs, int nJobs, i
   const JobDesc &J = jobs[j];
   SpacePrep p;
   SpaceRec r;
-  if (!prep_space(J.spaces[i - J.spaceBase], halfWidth, xMin, radius, J.cx, J.cy, J.cz, J.nProj, p, r))
+  if (!prep_space(load_space(J.spaces + (i - J.spaceBase)), halfWidth, xMin, radius, J.cx, J.cy, J.cz, J.nProj, p, r))
     atomicCAS(status, 0, FR_E_INVALID);
-  out[i] = p;
-  rec[i] = r;
+  store_record(out + i, p);
+  store_record(rec + i, r);
 }
 
-// As bin_kernel, for a batch: CTA c bins 8 bricks of the job whose binning groups hold c,
-// against that job's spaces only; counts, offsets and list entries are batch-wide.
+// As bin_kernel, for a batch: CTA c bins a row of the job whose binning CTAs hold c, against that
+// job's spaces only; counts, offsets and list entries are batch-wide.
 template<bool FILL>
 __global__ void __launch_bounds__(256) batch_bin_kernel(const JobDesc *__restrict__ jobs, int nJobs,
-  const SpacePrep *__restrict__ prep, int *__restrict__ counts, const int *__restrict__ offsets,
-  int *__restrict__ list, const int *__restrict__ status)
+  const SpacePrep *__restrict__ prep, BinBuffers buf)
 {
-  __shared__ SpacePrep tile[256];
-  __shared__ int hitIdx[256];
-  __shared__ int hitN, warpBase[8];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (FILL && *buf.status != 0) return;
   const int j = job_of(jobs, nJobs, int(blockIdx.x), [](const JobDesc &J) { return J.groupBase; });
   const JobDesc &J = jobs[j];
-  const int local = (int(blockIdx.x) - J.groupBase) * 8 + warp;
-  const bool active = local < J.nBricks;
-  const int b = J.brickBase + local;
-  if (FILL && *status != 0) return;
-  BinGeom g;
-  g.vx = J.vx;
-  g.vy = J.vy;
-  g.vz = J.vz;
-  g.nbx = J.nbx;
-  g.nby = J.nby;
-  g.nbz = J.nbz;
-  g.n_bricks = J.nBricks;
-  g.cx = J.cx;
-  g.cy = J.cy;
-  g.cz = J.cz;
-  int b0[3] = {}, b1[3] = {};
-  float a[3] = {}, e[3] = {};
-  if (active) brick_box(g, local, b0, b1, a, e);
-  int u0[3], u1[3];
-  float ua[3], ue[3];
-  const int first = (int(blockIdx.x) - J.groupBase) * 8;
-  union_box(g, first, min(8, J.nBricks - first), u0, u1, ua, ue);
-  int cnt[3] = { 0, 0, 0 };
-  if (FILL && active)
-    for (int d = 0; d < 3; ++d) cnt[d] = offsets[3 * b + d];
-  const int n = J.nSpaces;
-  SpacePrep next;
-  if (int(threadIdx.x) < n) next = load_prep(prep + J.spaceBase + threadIdx.x);
-  for (int base = 0; base < n; base += 256) {
-    __syncthreads();
-    if (base + int(threadIdx.x) < n) tile[threadIdx.x] = next;
-    __syncthreads();
-    if (base + 256 + int(threadIdx.x) < n) next = load_prep(prep + J.spaceBase + base + 256 + threadIdx.x);
-    const int m = min(256, n - base);
-    compact_tile_hits(tile, m, u0, u1, ua, ue, hitIdx, &hitN, warpBase);
-    if (!active) continue;
-    const int hn = hitN;
-    for (int r = 0; r < hn; r += 32) {
-      const int qq = r + lane;
-      bool hit = false;
-      int dir = 0, q = 0;
-      if (qq < hn) {
-        q = hitIdx[qq];
-        hit = brick_hit(tile[q], b0, b1, a, e);
-        dir = tile[q].dir;
-      }
-      for (int d = 0; d < 3; ++d) {
-        unsigned mask = __ballot_sync(0xffffffffu, hit && dir == d);
-        if (FILL && hit && dir == d) list[cnt[d] + __popc(mask & ((1u << lane) - 1u))] = J.spaceBase + base + q;
-        cnt[d] += __popc(mask);
-      }
-    }
-  }
-  if (!FILL && active && lane == 0)
-    for (int d = 0; d < 3; ++d) counts[3 * b + d] = cnt[d];
+  BinRow R;
+  R.g = { J.vx, J.vy, J.vz, J.nbx, J.nby, J.nbz, J.nBricks, J.cx, J.cy, J.cz };
+  const int rows = J.nby * J.nbz, c = int(blockIdx.x) - J.groupBase;
+  R.row = c % rows;
+  R.bx0 = c / rows * kRowBricks;
+  R.n = J.nSpaces;
+  R.brickBase = J.brickBase;
+  R.spaceBase = J.spaceBase;
+  R.job = j;
+  R.prep = prep + J.spaceBase;
+  bin_row<FILL>(R, buf.counts, buf.offsets, buf.list, buf);
 }
 
-// Single-CTA planner: exclusive scan of the (brick, direction) counts into list offsets,
-// then cuts every brick's list into work items (ItemSplit), bricks taken in `order` (heaviest
-// expected first).  Sets status = FR_E_CAPACITY instead of
-// overflowing the list or item buffers.  When the status is already set (a space with a
-// projection outside the FFT payload, or an earlier failure), the fill pass writes no lists,
-// so no work items are published either: the insertion then reads no list entry.
-__global__ void __launch_bounds__(1024) plan_kernel(BinGeom g, const int *__restrict__ counts,
-  int *__restrict__ offsets, const int *__restrict__ order, ItemSplit split, int64_t listCap,
-  int64_t itemsCap, WorkItem *__restrict__ items, int *__restrict__ nItems, int *__restrict__ status,
-  unsigned long long *__restrict__ stats, const JobDesc *__restrict__ jobs, int nJobs)
+// Exclusive prefix sum over the 1,024 threads of the CTA (every thread calls it); `total` in all.
+__device__ __forceinline__ long long block_scan(long long v, long long &total)
 {
-  __shared__ long long part[1024];
-  const int tid = threadIdx.x, T = blockDim.x;
-  const int prior = *status;  // read before this kernel writes it
-  // pass 1: offsets over 3*n_bricks counts
-  const int M = 3 * g.n_bricks;
-  const int per = (M + T - 1) / T;
-  long long s = 0;
-  for (int k = tid * per; k < min(M, (tid + 1) * per); ++k) s += counts[k];
-  part[tid] = s;
+  __shared__ long long warps[32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  long long incl = v;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const long long u = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += u;
+  }
+  __syncthreads();  // the previous scan's sums have been read
+  if (lane == 31) warps[warp] = incl;
   __syncthreads();
-  for (int off = 1; off < T; off <<= 1) {
-    long long v = tid >= off ? part[tid - off] : 0;
-    __syncthreads();
-    part[tid] += v;
-    __syncthreads();
+  if (warp == 0) {
+    long long w = warps[lane];
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const long long u = __shfl_up_sync(0xffffffffu, w, o);
+      if (lane >= o) w += u;
+    }
+    warps[lane] = w;
   }
-  long long run = part[tid] - s;
-  const long long total = part[T - 1];
-  for (int k = tid * per; k < min(M, (tid + 1) * per); ++k) {
-    offsets[k] = int(min(run, (long long)listCap));
-    run += counts[k];
+  __syncthreads();
+  total = warps[31];
+  return incl - v + (warp ? warps[warp - 1] : 0);
+}
+
+// Single-CTA planner: exclusive scan of the (brick, direction) counts into list offsets, then
+// the number of work items of every brick (ItemSplit) scanned into its first item, bricks taken
+// in `order` (heaviest expected first); the fill pass writes the items beside the lists.  Sets
+// status = FR_E_CAPACITY instead of overflowing the list or item buffers.  When the status is
+// already set (a space with a projection outside the FFT payload, or an earlier failure), the fill
+// pass writes no lists, so no work items are published either: the insertion then reads no list
+// entry.  Bound by the latency of its few dependent loads and barriers.
+__global__ void __launch_bounds__(1024) plan_kernel(int nBricks, BinBuffers b, ItemSplit split, bool first)
+{
+  __shared__ int longest;
+  const int tid = threadIdx.x, T = 1024;
+  const int prior = *b.status;  // read before this kernel writes it
+  // pass 1: offsets over 3 nBricks counts
+  const int M = 3 * nBricks;
+  const int per = (M + T - 1) / T, m0 = min(M, tid * per), m1 = min(M, m0 + per);
+  long long s = 0, total = 0;
+  for (int k = m0; k < m1; ++k) s += b.counts[k];
+  long long run = block_scan(s, total);
+  for (int k = m0; k < m1; ++k) {
+    b.offsets[k] = int(min(run, (long long)b.listCap));
+    run += b.counts[k];
   }
-  if (tid == 0) offsets[M] = int(min(total, (long long)listCap));
+  if (tid == 0) {
+    b.offsets[M] = int(min(total, (long long)b.listCap));
+    longest = 0;
+  }
   __syncthreads();
   // capacity of an item
   int itemCap = split.cap;
   if (split.want > 0) {  // uniform
-    __shared__ int longest;
-    if (tid == 0) longest = 0;
-    __syncthreads();
-    int len = 0;
-    if (split.perBrick > 0)
-      for (int b = tid; b < g.n_bricks; b += T) len = max(len, offsets[3 * b + 3] - offsets[3 * b]);
-    if (len > 0) atomicMax(&longest, len);
-    __syncthreads();
-    const long long shared = max((long long)split.least, (total + split.want - 1) / split.want);
-    const int whole = split.perBrick > 0 ? (longest + split.perBrick - 1) / split.perBrick : 0;
-    itemCap = int(min((long long)split.cap, max(shared, (long long)whole)));
-  }
-  // pass 2: items per brick in `order`
-  const int NB = g.n_bricks;
-  const int perb = (NB + T - 1) / T;
-  s = 0;
-  for (int k = tid * perb; k < min(NB, (tid + 1) * perb); ++k) {
-    int bb = order[k];
-    long long len = (long long)offsets[3 * bb + 3] - offsets[3 * bb];
-    s += (len + itemCap - 1) / itemCap;
-  }
-  __syncthreads();
-  part[tid] = s;
-  __syncthreads();
-  for (int off = 1; off < T; off <<= 1) {
-    long long v = tid >= off ? part[tid - off] : 0;
-    __syncthreads();
-    part[tid] += v;
-    __syncthreads();
-  }
-  run = part[tid] - s;
-  const long long totalItems = part[T - 1];
-  const bool fits = total <= listCap && totalItems <= itemsCap;
-  const bool ok = fits && prior == 0;
-  if (ok) {
-    for (int k = tid * perb; k < min(NB, (tid + 1) * perb); ++k) {
-      int bb = order[k];
-      int beg = offsets[3 * bb], end = offsets[3 * bb + 3];
-      int job = 0;  // batched plans: the job whose brick range holds bb
-      if (jobs) {
-        int lo = 0, hi = nJobs - 1;
-        while (lo < hi) {
-          const int mid = (lo + hi + 1) >> 1;
-          if (jobs[mid].brickBase <= bb) lo = mid;
-          else hi = mid - 1;
-        }
-        job = lo;
-      }
-      for (int q = beg; q < end; q += itemCap) {
-        WorkItem it;
-        it.brick = bb;
-        it.begin = q;
-        it.end = min(end, q + itemCap);
-        it.job = job;
-        items[run++] = it;
-      }
+    long long cap = max((long long)split.least, (total + split.want - 1) / split.want);
+    if (split.perBrick > 0) {
+      int len = 0;
+      for (int k = tid; k < nBricks; k += T) len = max(len, b.offsets[3 * k + 3] - b.offsets[3 * k]);
+      len = int(__reduce_max_sync(0xffffffffu, unsigned(len)));
+      if ((tid & 31) == 0 && len > 0) atomicMax(&longest, len);
+      __syncthreads();
+      cap = max(cap, (long long)((longest + split.perBrick - 1) / split.perBrick));
     }
+    itemCap = int(min((long long)split.cap, cap));
   }
+  // pass 2: first items, in `order`
+  const int perb = (nBricks + T - 1) / T, b0 = min(nBricks, tid * perb), b1 = min(nBricks, b0 + perb);
+  long long items = 0;
+  s = 0;
+  for (int k = b0; k < b1; ++k) {
+    const int bb = b.order[k];
+    s += (b.offsets[3 * bb + 3] - b.offsets[3 * bb] + itemCap - 1) / itemCap;
+  }
+  run = block_scan(s, items);
+  for (int k = b0; k < b1; ++k) {
+    const int bb = b.order[k];
+    b.itemStart[bb] = int(min(run, (long long)b.itemsCap));
+    run += (b.offsets[3 * bb + 3] - b.offsets[3 * bb] + itemCap - 1) / itemCap;
+  }
+  const bool fits = total <= b.listCap && items <= b.itemsCap;
+  const bool ok = fits && prior == 0;
   if (tid == 0) {
-    *nItems = ok ? int(totalItems) : 0;
-    if (!fits && prior == 0) *status = FR_E_CAPACITY;
-    stats[0] += (unsigned long long)total;
-    stats[1] += ok ? (unsigned long long)totalItems : 0ull;
-    stats[2] += 1ull;
+    *b.itemCap = itemCap;
+    *b.workCounter = 0;
+    *b.nItems = ok ? int(items) : 0;
+    if (!fits && prior == 0) *b.status = FR_E_CAPACITY;
+    b.stats[0] = (first ? 0ull : b.stats[0]) + (unsigned long long)total;
+    b.stats[1] = (first ? 0ull : b.stats[1]) + (ok ? (unsigned long long)items : 0ull);
+    b.stats[2] = (first ? 0ull : b.stats[2]) + 1ull;
   }
 }
 
@@ -590,16 +467,11 @@ cudaError_t launch_batch_binning(const JobDesc *jobs, int nJobs, int totalSpaces
   const float hw = fast ? 2.5f : radius + 1e-3f;
   const float xmin = fast ? -1e-3f : -radius - 1e-3f;
   if (totalSpaces > 0)
-    batch_prep_kernel<<<(totalSpaces + 255) / 256, 256, 0, st>>>(jobs, nJobs, totalSpaces, hw, xmin, radius,
+    batch_prep_kernel<<<(totalSpaces + 63) / 64, 64, 0, st>>>(jobs, nJobs, totalSpaces, hw, xmin, radius,
       b.prep, b.rec, b.status);
-  prefer_max_shared(batch_bin_kernel<false>);
-  prefer_max_shared(batch_bin_kernel<true>);
-  batch_bin_kernel<false><<<totalGroups, 256, 0, st>>>(jobs, nJobs, b.prep, b.counts, nullptr, nullptr, b.status);
-  BinGeom g{};
-  g.n_bricks = totalBricks;
-  plan_kernel<<<1, 1024, 0, st>>>(g, b.counts, b.offsets, b.order, split, b.listCap, b.itemsCap, b.items,
-    b.nItems, b.status, b.stats, jobs, nJobs);
-  batch_bin_kernel<true><<<totalGroups, 256, 0, st>>>(jobs, nJobs, b.prep, nullptr, b.offsets, b.list, b.status);
+  batch_bin_kernel<false><<<totalGroups, 256, 0, st>>>(jobs, nJobs, b.prep, b);
+  plan_kernel<<<1, 1024, 0, st>>>(totalBricks, b, split, true);
+  batch_bin_kernel<true><<<totalGroups, 256, 0, st>>>(jobs, nJobs, b.prep, b);
   return cudaGetLastError();
 }
 
@@ -687,7 +559,7 @@ __global__ void batch_band_kernel(const JobDesc *__restrict__ jobs, int nJobs, i
 
 // Two 256-thread CTAs per SM: enough loads in flight to run near the copy bandwidth, and room
 // left on every SM for the binning kernels that run beside the copy on the other stream
-// (prefer_max_shared).
+// (prefer_shared_carveout).
 static int band_blocks(int64_t units)
 {
   int dev = 0, sms = 148;
@@ -700,8 +572,6 @@ cudaError_t launch_band_projections(const void *src, void *dst, int64_t n, int f
 {
   if (n <= 0) return cudaSuccess;
   const int blocks = band_blocks(n * ((fftY + 3) / 4));
-  prefer_max_shared(band_kernel<float2>);
-  prefer_max_shared(band_kernel<uint32_t>);
   if (elemBytes == 8)
     band_kernel<float2><<<blocks, 256, 0, st>>>(static_cast<const float2 *>(src), static_cast<float2 *>(dst), n, fftX,
       fftY);
@@ -715,29 +585,56 @@ cudaError_t launch_batch_band(const JobDesc *jobs, int nJobs, int64_t totalUnits
 {
   if (totalUnits <= 0) return cudaSuccess;
   const int blocks = band_blocks(totalUnits);
-  prefer_max_shared(batch_band_kernel<float2>);
-  prefer_max_shared(batch_band_kernel<uint32_t>);
   if (elemBytes == 8) batch_band_kernel<float2><<<blocks, 256, 0, st>>>(jobs, nJobs, totalUnits);
   else batch_band_kernel<uint32_t><<<blocks, 256, 0, st>>>(jobs, nJobs, totalUnits);
   return cudaGetLastError();
 }
 
 cudaError_t launch_binning(const BinGeom &g, const fr_traverse_space *spaces, int n, int nProj,
-  bool fast, float radius, const BinBuffers &b, const ItemSplit &split, cudaStream_t st)
+  bool fast, float radius, const BinBuffers &b, const ItemSplit &split, bool first, cudaStream_t st)
 {
   const float hw = fast ? 2.5f : radius + 1e-3f;
   const float xmin = fast ? -1e-3f : -radius - 1e-3f;
+  space_prep_kernel<<<(n + 63) / 64, 64, 0, st>>>(spaces, n, hw, xmin, radius, g.cx, g.cy, g.cz, nProj, b.prep, b.rec,
+    b.status);
+  const int blocks = bin_groups(g.nbx, g.nby, g.nbz);
+  bin_kernel<false><<<blocks, 256, 0, st>>>(g, b.prep, n, b);
+  plan_kernel<<<1, 1024, 0, st>>>(g.n_bricks, b, split, first);
+  bin_kernel<true><<<blocks, 256, 0, st>>>(g, b.prep, n, b);
+  return cudaGetLastError();
+}
+
+// The band copy, the binning and the insertion all ask for the largest shared-memory carve-out,
+// so that an SM running copy CTAs (which need no shared memory) can take binning CTAs beside
+// them instead of waiting for the copy to end.
+template<typename K> static void prefer_max_shared(K *kernel)
+{
+  if (cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared)
+      != cudaSuccess)
+    cudaGetLastError();  // a hint only
+}
+
+void prefer_shared_carveout()
+{
   prefer_max_shared(space_prep_kernel);
   prefer_max_shared(bin_kernel<false>);
   prefer_max_shared(bin_kernel<true>);
-  space_prep_kernel<<<(n + 255) / 256, 256, 0, st>>>(spaces, n, hw, xmin, radius, g.cx, g.cy, g.cz, nProj,
-    b.prep, b.rec, b.status);
-  const int blocks = (g.n_bricks + 7) / 8;
-  bin_kernel<false><<<blocks, 256, 0, st>>>(g, b.prep, n, b.counts, nullptr, nullptr, b.status);
-  plan_kernel<<<1, 1024, 0, st>>>(g, b.counts, b.offsets, b.order, split, b.listCap, b.itemsCap,
-    b.items, b.nItems, b.status, b.stats, nullptr, 0);
-  bin_kernel<true><<<blocks, 256, 0, st>>>(g, b.prep, n, nullptr, b.offsets, b.list, b.status);
-  return cudaGetLastError();
+  prefer_max_shared(batch_bin_kernel<false>);
+  prefer_max_shared(batch_bin_kernel<true>);
+  prefer_max_shared(band_kernel<float2>);
+  prefer_max_shared(band_kernel<uint32_t>);
+  prefer_max_shared(batch_band_kernel<float2>);
+  prefer_max_shared(batch_band_kernel<uint32_t>);
+}
+
+void set_misc(BinBuffers &b, int *misc)
+{
+  b.itemStart = b.counts;  // read once the counts have been
+  b.nItems = misc;
+  b.status = misc + kMiscStatus;
+  b.workCounter = misc + 2;
+  b.itemCap = misc + 3;
+  b.stats = reinterpret_cast<unsigned long long *>(misc + kMiscStats);
 }
 
 // Few spaces on few bricks left most brick groups idle: a group inserts one entry of its item

@@ -26,14 +26,17 @@ struct BinGeom {
 struct BinBuffers {
   SpacePrep *prep;        // [chunk capacity]
   SpaceRec *rec;          // [chunk capacity]
-  int *counts;            // [3 * n_bricks]
+  int *counts;            // [3 * n_bricks]; after the plan itemStart's memory
   int *offsets;           // [3 * n_bricks + 1]
   int *list;              // [listCap] space indices, grouped by (brick, direction)
   const int *order;       // [n_bricks] brick visiting order (heaviest expected first)
   WorkItem *items;        // [itemsCap]
+  int *itemStart;         // [n_bricks] first work item of each brick
   int *nItems;            // [1]
   int *status;            // [1] sticky FR_E_* of device-side failures
-  unsigned long long *stats;  // [4] pairs, items, chunks
+  int *workCounter;       // [1] next work item of the insertion
+  int *itemCap;           // [1] list entries per work item
+  unsigned long long *stats;  // [4] pairs, items, chunks of the call
   int64_t listCap;
   int64_t itemsCap;
 };
@@ -146,11 +149,21 @@ cudaError_t launch_band_projections(const void *src, void *dst, int64_t n, int f
 // The same for every job of a batch: job j's projections go from its `src` to its `fft`, its
 // bands numbered from its `unitBase` (totalUnits bands in all).
 cudaError_t launch_batch_band(const JobDesc *jobs, int nJobs, int64_t totalUnits, int elemBytes, cudaStream_t st);
-// `split`: see ItemSplit.
+// Engine scratch's small words, one device block mirrored by one pinned host block.
+constexpr int kMiscStatus = 1, kMiscStats = 4;  // word indices: status; stats (4 x 64 bits)
+constexpr size_t kMiscBytes = 48;
+void set_misc(BinBuffers &b, int *misc);
+// Sets the carve-out preference of the kernels that run beside one another (fr_create).
+void prefer_shared_carveout();
+
+// Binning and planning of one chunk of a call's spaces (`first`: its first chunk, which starts the
+// call's statistics).  `split`: see ItemSplit.
 cudaError_t launch_binning(const BinGeom &g, const fr_traverse_space *spaces, int n, int nProj,
-  bool fast, float radius, const BinBuffers &b, const ItemSplit &split, cudaStream_t st);
+  bool fast, float radius, const BinBuffers &b, const ItemSplit &split, bool first, cudaStream_t st);
+// Brick rows of a volume the binning takes one CTA for (fr_binning.cuh, bin_row).
+__host__ __device__ inline int bin_groups(int nbx, int nby, int nbz) { return (nbx + 31) / 32 * nby * nbz; }
 // Binning of a batch: jobs (device job table, nJobs entries) with totalSpaces spaces,
-// totalBricks bricks and totalGroups 8-brick binning groups in all.
+// totalBricks bricks and totalGroups binning CTAs (bin_groups) in all.
 cudaError_t launch_batch_binning(const JobDesc *jobs, int nJobs, int totalSpaces, int totalBricks,
   int totalGroups, bool fast, float radius, const BinBuffers &b, const ItemSplit &split, cudaStream_t st);
 cudaError_t launch_insert(const InsertParams &P, const InsertConfig &cfg, int grid, cudaStream_t st);

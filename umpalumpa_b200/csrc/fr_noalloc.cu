@@ -160,8 +160,6 @@ extern "C" int fr_insert_noalloc(int device, void *stream, const fr_dims *d, con
   size_t off = 0;
   const size_t oMisc = off;
   off += 256;
-  const size_t oStats = off;
-  off += 256;
   const size_t oCounts = off;
   off += align256(size_t(3) * g.n_bricks * sizeof(int));
   const size_t oOffsets = off;
@@ -202,16 +200,12 @@ extern "C" int fr_insert_noalloc(int device, void *stream, const fr_dims *d, con
   bb.list = reinterpret_cast<int *>(sb + oList);
   bb.order = reinterpret_cast<const int *>(sb + oOrder);
   bb.items = reinterpret_cast<frb::WorkItem *>(sb + oItems);
-  bb.nItems = misc;
-  bb.status = misc + 1;
-  int *workCounter = misc + 2;
-  bb.stats = reinterpret_cast<unsigned long long *>(sb + oStats);
+  frb::set_misc(bb, misc);
   bb.listCap = listCap;
   bb.itemsCap = itemsCap;
 
   // the array keeps the previous call's contents: clear what must start at zero
   cudaError_t e = cudaMemsetAsync(misc, 0, 256, st);
-  if (e == cudaSuccess) e = cudaMemsetAsync(bb.stats, 0, 256, st);
   if (e == cudaSuccess) {
     noalloc_order_kernel<<<1, 1024, 0, st>>>(g, reinterpret_cast<int *>(sb + oOrder));
     e = cudaGetLastError();
@@ -244,7 +238,7 @@ extern "C" int fr_insert_noalloc(int device, void *stream, const fr_dims *d, con
   P.offsets = bb.offsets;
   P.items = bb.items;
   P.nItems = bb.nItems;
-  P.workCounter = workCounter;
+  P.workCounter = bb.workCounter;
   P.table = kaiserTable ? kaiser : table;
   P.tableElems = kaiserTable ? frb::kKaiserTableElems
                              : int(s->interpolation == FR_INTERPOLATION_LOOKUP ? d->table_elems : 0);
@@ -269,8 +263,7 @@ extern "C" int fr_insert_noalloc(int device, void *stream, const fr_dims *d, con
   P.cz = g.cz;
   for (uint64_t s0 = 0; s0 < nSpaces && e == cudaSuccess; s0 += uint64_t(chunk)) {
     const int n = int(std::min<uint64_t>(uint64_t(chunk), nSpaces - s0));
-    e = frb::launch_binning(g, spaces + s0, n, int(nProj), cfg.fast, s->blob_radius, bb, split, st);
-    if (e == cudaSuccess) e = cudaMemsetAsync(workCounter, 0, sizeof(int), st);
+    e = frb::launch_binning(g, spaces + s0, n, int(nProj), cfg.fast, s->blob_radius, bb, split, s0 == 0, st);
     if (e == cudaSuccess) e = frb::launch_insert(P, cfg, sms * occ, st);
   }
   int status = 0;
