@@ -76,3 +76,13 @@ def test_axis_aligned_planes(cuda):
     rots = np.ascontiguousarray(rots.astype(np.float32))
     spaces = oracle.traverse_spaces(rots, box // 2, box, box, box)
     assert max(_run(cuda, box, fft, spaces, 1.9)) <= TOL
+
+
+@pytest.mark.parametrize("box,radius", [(4, 1.9), (6, 1.9), (10, 3.9)])
+def test_half_planes_smaller_than_the_window(cuda, box, radius):
+    n = 20
+    fft, rots = synthetic.make_job(box, n, seed=box, snr=0.1)
+    spaces = oracle.traverse_spaces(rots, box // 2, box, box, box, radius=radius)
+    for layout in (0, 1):
+        assert max(_run(cuda, box, fft, spaces, radius, layout)) <= TOL
+        assert max(_run(cuda, box, fft, spaces, radius, layout, table=False)) <= TOL

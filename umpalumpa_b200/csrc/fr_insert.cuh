@@ -26,11 +26,11 @@
 //
 // What bounds it (lookup, FP32, banded, 1,537-20,000 projections at box 256): the L1/shared data
 // path (117 wavefronts per step of 32 voxels: 60 pixel gathers, 34 table lookups, 13 accumulators)
-// at 73 % and instruction issue at 66 %, with the 24 warps that shared memory and registers
+// at 79 % and instruction issue at 66 %, with the 24 warps that shared memory and registers
 // allow.  Against steps that start anew for every projection (26 of 32 lanes filled, the source
 // columns found by a binary search over shuffles), with one voxel body per direction instead of
-// one for all: 19 % fewer instructions and 13 % fewer wavefronts; 20,000 projections
-// 45.8 -> 37.5 ms.
+// one for all: 17 % fewer instructions and 14 % fewer wavefronts; 20,000 projections
+// 45.8 -> 36.3 ms (the whole call).
 //
 // Half-plane layouts (BANDED): the caller's row-major half-planes, or the same pixels in bands
 // of four rows stored column by column (pixel (y, x) at (y / 4) * bandStride + 4 x + y % 4,
@@ -203,10 +203,12 @@ __device__ __forceinline__ bool voxel_blob(const InsertParams &P, const JobGeom 
   const float rSq = mul_(r, r);
   const float zSq = mul_(qz, qz);
   // The reference's rejection tests -- outside the frequency sphere (integer-valued: exact),
-  // behind the image, off the slab -- and those no pixel lies within the blob radius of (also
-  // rejects non-finite coordinates), as one predicate.
-  const bool inside = !(px * px + py * py + pz * pz > s.maxDist2) & !(qx < -r) & !(zSq > rSq)
-                      & (qx <= float(G.fftX) + r) & (qy >= -r) & (qy <= float(G.fftY) + r);
+  // behind the image, off the slab -- as one predicate.  A voxel beyond the image's other edges, or
+  // at a non-finite coordinate, finds no pixel within the radius in its window (which lies inside
+  // the image whatever the coordinate is) and adds zeros; GENERIC windows are not shifted into
+  // the image, so there it is rejected.
+  bool inside = !(px * px + py * py + pz * pz > s.maxDist2) & !(qx < -r) & !(zSq > rSq);
+  if (GENERIC) inside = inside & (qx <= float(G.fftX) + r) & (qy >= -r) & (qy <= float(G.fftY) + r);
   if (!inside) return false;
   // The TAPS x TAPS window starts at (ceil(qx - r), ceil(qy - r)) shifted into the image, so
   // it covers the reference's clamped blob box [max(ceil(q - r), 0), min(floor(q + r), X-1)]
@@ -468,9 +470,14 @@ __device__ __forceinline__ void insert_blobs(const InsertParams &P, const JobGeo
         ok = voxel_blob<MODE, TAPS, STORAGE, false, BANDED>(P, G, s, img, bandStride, scale, lut, px, py, pz, v, w);
     }
     const int slot = acc_slot(voxel & 4095);
-    for (int p = 0; p < parts; ++p) {
-      if (ok && voxel >> 12 == p) acc_add<KAHAN>(A, slot, v, w);
-      __syncwarp();  // the next entry or step may revisit these voxels from other lanes
+    if (parts == 1) {  // two steps of three
+      if (ok) acc_add<KAHAN>(A, slot, v, w);
+      __syncwarp();  // the next step may revisit these voxels from other lanes
+    } else {
+      for (int p = 0; p < parts; ++p) {
+        if (ok && voxel >> 12 == p) acc_add<KAHAN>(A, slot, v, w);
+        __syncwarp();  // as may the next entry
+      }
     }
     n = 0;
     parts = 0;
