@@ -833,21 +833,21 @@ def run_prep(a):
                                f"{'complex64' if storage == 0 else a.storage + ' complex + fp32 scale'} half-planes, "
                                "normalise + centre + shift (the example driver's AFP settings)",
                    "l2": f"no flush: {n * 4 * box * box / 1e9:.1f} GB of images exceed L2", "parallelism": "single GPU"},
-        "fft_route": "fused (the engine's own FFT + processing in one kernel)" if box in (64, 128, 256)
+        "fft_route": "fused (the engine's own FFT + processing in one kernel)" if box in (64, 96, 128, 192, 256, 320, 384)
                      else "cuFFT R2C + one processing pass",
         "cufft_route": {"value": n / (cufft_ms / 1000.0), "ms_per_step": cufft_ms,
                         "rel_l2_vs_fused": route_diff},
         "unfused_torch": None if unfused_ms is None else {"value": n / (unfused_ms / 1000.0), "ms_per_step": unfused_ms},
         "pipeline": pipeline,
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
-                     "traffic": None, "kernel": "frb::prepfft::prep_fft_kernel" if box in (64, 128, 256)
+                     "traffic": None, "kernel": "frb::prepfft::prep_fft_kernel" if box in (64, 96, 128, 192, 256, 320, 384)
                      else "cuFFT R2C + frb prep_kernel", "peak_source": src,
                      "algorithmic_bytes_per_image": bytes_per_image},
         "rel_l2_vs_oracle": err,
         "cpu_baseline": {"value": take / cpu_s, "unit": "images/s", "cores": 1, "kind": "port",
                          "sample": f"{take} images, numpy FFT (double) + the restated processing"},
         "chunk": a.prep_chunk or prep_chunk(box),
-        "gpu_launches": 1 if box in (64, 128, 256) else
+        "gpu_launches": 1 if box in (64, 96, 128, 192, 256, 320, 384) else
                         2 * ((n + (a.prep_chunk or prep_chunk(box)) - 1) // (a.prep_chunk or prep_chunk(box))),
         "clocks": clk.summary(),
     }
