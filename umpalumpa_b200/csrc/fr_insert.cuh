@@ -202,13 +202,15 @@ __device__ __forceinline__ bool voxel_blob(const InsertParams &P, const JobGeom 
   const float qy = add_(qy0, float(G.cy));
   const float rSq = mul_(r, r);
   const float zSq = mul_(qz, qz);
-  // The reference's rejection tests -- outside the frequency sphere (integer-valued: exact),
-  // behind the image, off the slab -- as one predicate.  A voxel beyond the image's other edges, or
-  // at a non-finite coordinate, finds no pixel within the radius in its window (which lies inside
-  // the image whatever the coordinate is) and adds zeros; GENERIC windows are not shifted into
-  // the image, so there it is rejected.
-  bool inside = !(px * px + py * py + pz * pz > s.maxDist2) & !(qx < -r) & !(zSq > rSq);
-  if (GENERIC) inside = inside & (qx <= float(G.fftX) + r) & (qy >= -r) & (qy <= float(G.fftY) + r);
+  // Outside the frequency sphere (integer-valued: exact), behind the image or off the slab, as
+  // the reference rejects; and beyond the image's other edges, where no pixel lies within the
+  // radius (which also rejects non-finite coordinates).  One predicate: the tests are independent.
+  // The last three cost 0.3-1.1 % where no voxel lies out there (box 256 x 20,000 36.3 -> 36.4 ms),
+  // but keep a voxel that can only add zeros out of the taps -- 2,000 half-planes cropped to
+  // 33 x 64 into box 256 take 1.77 ms with them, 2.84 without -- and out of the sums, where the
+  // zeros times an infinite or NaN weight would be NaN.
+  const bool inside = !(px * px + py * py + pz * pz > s.maxDist2) & !(qx < -r) & !(zSq > rSq)
+                      & (qx <= float(G.fftX) + r) & (qy >= -r) & (qy <= float(G.fftY) + r);
   if (!inside) return false;
   // The TAPS x TAPS window starts at (ceil(qx - r), ceil(qy - r)) shifted into the image, so
   // it covers the reference's clamped blob box [max(ceil(q - r), 0), min(floor(q + r), X-1)]
