@@ -144,6 +144,7 @@ struct BinRow {
   BinGeom g;
   int row, bx0, n;            // n spaces from prep
   int brickBase, spaceBase, job;
+  int cap;                    // the items' full capacity (ItemSplit)
   const SpacePrep *prep;
 };
 
@@ -223,10 +224,11 @@ __device__ __forceinline__ void bin_row(const BinRow &R, int *__restrict__ count
     if (tid < 3 * nb) counts[3 * first + tid] = count;
     return;
   }
-  // the bricks' work items: at most `cap` list entries each, from the plan's first item on
-  const int cap = *buf.itemCap;
+  // the bricks' work items: at most the plan's capacity each (Kahan: R.cap where not cut), from the
+  // plan's first item on
   for (int b = warp; b < nb; b += 8) {
     const int brick = first + b, beg = offsets[3 * brick], end = offsets[3 * brick + 3], item = buf.itemStart[brick];
+    const int cap = buf.merge.slot && buf.merge.slot[brick] < 0 ? R.cap : *buf.itemCap;
     for (int q = lane; beg + q * cap < end; q += 32)
       buf.items[item + q] = { brick, beg + q * cap, min(end, beg + (q + 1) * cap), R.job };
   }

@@ -236,6 +236,30 @@ static frb::ItemSplit handle_split(const fr_handle *h)
   return frb::item_split(h->launch.item_capacity, h->grid * frb::insert_groups(h->cfg), h->cfg);
 }
 
+// The Kahan handle's brick sums, for its split and at most nBricks bricks.  Where their memory
+// cannot be had, bricks are not cut.
+static cudaError_t alloc_merge(fr_handle *h, int64_t nBricks)
+{
+  const int slots = frb::merge_slots(handle_split(h), nBricks);
+  if (slots == 0 && !h->cfg.kahan) return cudaSuccess;
+  const size_t sumBytes = size_t(slots) * frb::kMergeSlotBytes, brickBytes = align256(size_t(nBricks) * sizeof(int));
+  frb::MergeBuffers &m = h->bb.merge;
+  m.slots = slots;
+  h->merge_bytes = sumBytes + 2 * brickBytes;
+  if (cudaMalloc(&h->merge, h->merge_bytes) != cudaSuccess) {
+    cudaGetLastError();
+    m.slots = 0;
+    h->merge_bytes = 2 * brickBytes;
+    const cudaError_t e = cudaMalloc(&h->merge, h->merge_bytes);
+    if (e != cudaSuccess) return e;
+  }
+  char *base = static_cast<char *>(h->merge);
+  m.slot = reinterpret_cast<int *>(base);
+  m.left = reinterpret_cast<int *>(base + brickBytes);
+  m.sums = reinterpret_cast<double *>(base + 2 * brickBytes);
+  return cudaMemsetAsync(h->merge, 0, h->merge_bytes, h->stream);
+}
+
 int frb::batch_device_status(const fr_handle *h) { return h && h->host_status ? h->host_status[0] : FR_E_INVALID; }
 
 static cudaEvent_t next_event(fr_handle *h, int &idx)
@@ -347,6 +371,10 @@ int fr_cleanup(fr_handle *h)
     if (h->band_stream) cudaStreamSynchronize(h->band_stream);
   }
   if (h->scratch) cudaFree(h->scratch);
+  if (h->merge) cudaFree(h->merge);
+  h->merge = nullptr;
+  h->merge_bytes = 0;
+  h->bb.merge = {};
   if (h->band) cudaFree(h->band);
   h->band = nullptr;
   h->band_bytes = 0;
@@ -528,6 +556,7 @@ int fr_init(fr_handle *h, const fr_dims *d, const fr_settings *s)
   frb::set_misc(bb, misc);
   bb.listCap = listCap;
   bb.itemsCap = itemsCap;
+  FR_CUDA(alloc_merge(h, g.n_bricks));
   FR_CUDA(cudaMemcpyAsync(base + oOrder, order.data(), order.size() * sizeof(int), cudaMemcpyHostToDevice, h->stream));
   FR_CUDA(cudaMemsetAsync(misc, 0, 64, h->stream));
   h->kaiser_table = nullptr;
@@ -543,7 +572,7 @@ int fr_init(fr_handle *h, const fr_dims *d, const fr_settings *s)
 
 uint64_t fr_used_bytes(const fr_handle *h)
 {
-  return h ? uint64_t(h->scratch_bytes + h->slots[0].bytes + h->slots[1].bytes + h->band_bytes) : 0;
+  return h ? uint64_t(h->scratch_bytes + h->merge_bytes + h->slots[0].bytes + h->slots[1].bytes + h->band_bytes) : 0;
 }
 
 int fr_get_launch_params(const fr_handle *h, fr_launch_params *out)
@@ -734,6 +763,7 @@ int fr_execute(fr_handle *h, const void *fft, const float *scales, uint64_t nPro
   P.items = h->bb.items;
   P.nItems = h->bb.nItems;
   P.workCounter = h->bb.workCounter;
+  P.merge = h->bb.merge;
   set_table(P, h, table, h->dims.table_elems);
   P.lutInSmem = frb::insert_lut_in_smem(h->cfg, P.tableElems);
   P.genericTaps = int(h->dims.fft_x) < h->cfg.taps || int(h->dims.fft_y) < h->cfg.taps || P.tableElems > frb::kLutSmemMax;
@@ -876,6 +906,7 @@ int fr_batch_init(fr_handle *h, const fr_batch_limits *lim, const fr_settings *s
   frb::set_misc(bb, misc);
   bb.listCap = listCap;
   bb.itemsCap = itemsCap;
+  FR_CUDA(alloc_merge(h, nb));
   h->d_jobs = reinterpret_cast<frb::JobDesc *>(base + oJobs);
   for (int k = 0; k < 2; ++k) {
     FR_CUDA(cudaHostAlloc(reinterpret_cast<void **>(&h->h_jobs_set[k]), size_t(lim->max_jobs) * sizeof(frb::JobDesc),
@@ -925,6 +956,7 @@ static int enqueue_batch(fr_handle *h, int nJobs, int totalSpaces, int totalBric
   P.items = h->bb.items;
   P.nItems = h->bb.nItems;
   P.workCounter = h->bb.workCounter;
+  P.merge = h->bb.merge;
   set_table(P, h, table, h->blim.table_elems);
   P.lutInSmem = frb::insert_lut_in_smem(h->cfg, P.tableElems);
   P.c = h->constants;

@@ -43,6 +43,8 @@ struct fr_handle {
   void *scratch = nullptr;
   size_t scratch_bytes = 0;
   frb::BinBuffers bb{};
+  void *merge = nullptr;                      // bb.merge's memory (Kahan accumulation)
+  size_t merge_bytes = 0;
   int *host_misc = nullptr;                   // pinned mirror of the scratch's small words (set_misc)
   int *host_status = nullptr;                 // in it: the status
   unsigned long long *host_stats = nullptr;   // in it: the call's counters

@@ -557,6 +557,7 @@ __global__ void __launch_bounds__(kThreads *Groups<KAHAN, FAST>::value, 1) inser
   extern __shared__ float4 smem4[];
   float *smem = reinterpret_cast<float *>(smem4);
   __shared__ int sItem[kMaxGroups];
+  __shared__ int sLast[KAHAN ? kMaxGroups : 1];  // the item ends a merged brick
   __shared__ uint16_t sVoxels[FAST ? 1 : kMaxGroups * (kThreads / 32)][kVoxelList];
   // Batched launches: the current job's geometry, one copy per group in shared memory.  Held
   // in registers (as the single-job kernel may, where the values are constant operands of the
@@ -613,8 +614,14 @@ __global__ void __launch_bounds__(kThreads *Groups<KAHAN, FAST>::value, 1) inser
         insert_blobs<MODE, TAPS, STORAGE, KAHAN, JOBS, BANDED>(P, G, A, lut, sVoxels[threadIdx.x >> 5], ox, oy, oz, dir, warp, lane, e0, e1);
       group_sync(group);  // the next direction maps warps to other voxels
     }
-    // add the brick into the caller's volume and clear it (an item has at least one entry, so a
+    // add the brick into the caller's volume -- Kahan: a cut brick into its FP64 sums, which the
+    // last of its items adds to the volume -- and clear it (an item has at least one entry, so a
     // barrier lies between the reads of sItem above and its new value)
+    double *sums = nullptr;
+    if (KAHAN && P.merge.slot) {
+      const int slot = P.merge.slot[it.brick];  // uniform across the group
+      if (slot >= 0) sums = P.merge.sums + size_t(slot) * (3 * kBrickVox);
+    }
     for (int lin = tid; lin < kBrickVox; lin += kThreads) {
       const int i = acc_slot(lin);
       float2 v = A.v[i];
@@ -623,11 +630,19 @@ __global__ void __launch_bounds__(kThreads *Groups<KAHAN, FAST>::value, 1) inser
       A.w[i] = 0.f;
       if (KAHAN) {
         const float2 c = __bfloat1622float2(A.cv[i]);
-        v.x = __fsub_rn(v.x, c.x);
-        v.y = __fsub_rn(v.y, c.y);
-        w = __fsub_rn(w, __bfloat162float(A.cw[i]));
+        const float cw = __bfloat162float(A.cw[i]);
         A.cv[i] = __floats2bfloat162_rn(0.f, 0.f);
         A.cw[i] = __float2bfloat16_rn(0.f);
+        if (sums) {
+          const double x = double(v.x) - c.x, y = double(v.y) - c.y, z = double(w) - cw;
+          if (x != 0.0) atomicAdd(sums + lin, x);
+          if (y != 0.0) atomicAdd(sums + kBrickVox + lin, y);
+          if (z != 0.0) atomicAdd(sums + 2 * kBrickVox + lin, z);
+          continue;
+        }
+        v.x = __fsub_rn(v.x, c.x);
+        v.y = __fsub_rn(v.y, c.y);
+        w = __fsub_rn(w, cw);
       }
       const int X = ox + (lin & 15), Y = oy + (lin >> 4 & 15), Z = oz + (lin >> 8);
       if (X >= G.vx || Y >= G.vy || Z >= G.vz) continue;
@@ -635,6 +650,35 @@ __global__ void __launch_bounds__(kThreads *Groups<KAHAN, FAST>::value, 1) inser
       const size_t g = (size_t(Z) * G.vy + Y) * G.vx + X;
       atomicAdd(reinterpret_cast<float2 *>(G.volume) + g, v);
       atomicAdd(G.weight + g, w);
+    }
+    if (KAHAN && sums) {
+      __threadfence();    // this thread's adds before the count of the items still to come
+      group_sync(group);
+      if (tid == 0) sLast[group] = atomicSub(P.merge.left + it.brick, 1) == 1;
+      group_sync(group);
+      if (sLast[group]) {
+        __threadfence();  // the other items' adds after the count
+        // bound by the latency of its loads: four voxels in flight per thread (one: 5 us more
+        // per call, eight: the same)
+        constexpr int kAhead = 4;
+        for (int l0 = tid; l0 < kBrickVox; l0 += kAhead * kThreads) {
+          double m[kAhead][3];
+#pragma unroll
+          for (int k = 0; k < 3 * kAhead; ++k)
+            m[k / 3][k % 3] = __ldcg(sums + (k % 3) * kBrickVox + l0 + (k / 3) * kThreads);
+#pragma unroll
+          for (int k = 0; k < kAhead; ++k) {
+            const int lin = l0 + k * kThreads;
+            const float x = float(m[k][0]), y = float(m[k][1]), z = float(m[k][2]);
+            sums[lin] = sums[kBrickVox + lin] = sums[2 * kBrickVox + lin] = 0.0;
+            const int X = ox + (lin & 15), Y = oy + (lin >> 4 & 15), Z = oz + (lin >> 8);
+            if (X >= G.vx || Y >= G.vy || Z >= G.vz || (x == 0.f && y == 0.f && z == 0.f)) continue;
+            const size_t g = (size_t(Z) * G.vy + Y) * G.vx + X;
+            atomicAdd(reinterpret_cast<float2 *>(G.volume) + g, make_float2(x, y));
+            atomicAdd(G.weight + g, z);
+          }
+        }
+      }
     }
     if (tid == 0) sItem[group] = next;
   }

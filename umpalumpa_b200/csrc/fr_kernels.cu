@@ -257,7 +257,8 @@ __global__ void space_prep_kernel(const fr_traverse_space *__restrict__ spaces, 
 // The lists of one row of bricks (bin_row).  FILL does nothing once the status is set: the plan
 // then publishes no items, and the lists would not be read.
 template<bool FILL>
-__global__ void __launch_bounds__(256) bin_kernel(BinGeom g, const SpacePrep *__restrict__ prep, int n, BinBuffers b)
+__global__ void __launch_bounds__(256) bin_kernel(BinGeom g, const SpacePrep *__restrict__ prep, int n, BinBuffers b,
+  int cap)
 {
   if (FILL && *b.status != 0) return;
   BinRow R;
@@ -267,6 +268,7 @@ __global__ void __launch_bounds__(256) bin_kernel(BinGeom g, const SpacePrep *__
   R.bx0 = blockIdx.x / rows * kRowBricks;
   R.n = n;
   R.brickBase = R.spaceBase = R.job = 0;
+  R.cap = cap;
   R.prep = prep;
   bin_row<FILL>(R, b.counts, b.offsets, b.list, b);
 }
@@ -305,7 +307,7 @@ __global__ void batch_prep_kernel(const JobDesc *__restrict__ jobs, int nJobs, i
 // job's spaces only; counts, offsets and list entries are batch-wide.
 template<bool FILL>
 __global__ void __launch_bounds__(256) batch_bin_kernel(const JobDesc *__restrict__ jobs, int nJobs,
-  const SpacePrep *__restrict__ prep, BinBuffers buf)
+  const SpacePrep *__restrict__ prep, BinBuffers buf, int cap)
 {
   if (FILL && *buf.status != 0) return;
   const int j = job_of(jobs, nJobs, int(blockIdx.x), [](const JobDesc &J) { return J.groupBase; });
@@ -319,6 +321,7 @@ __global__ void __launch_bounds__(256) batch_bin_kernel(const JobDesc *__restric
   R.brickBase = J.brickBase;
   R.spaceBase = J.spaceBase;
   R.job = j;
+  R.cap = cap;
   R.prep = prep + J.spaceBase;
   bin_row<FILL>(R, buf.counts, buf.offsets, buf.list, buf);
 }
@@ -358,6 +361,7 @@ __device__ __forceinline__ long long block_scan(long long v, long long &total)
 // already set (a space with a projection outside the FFT payload, or an earlier failure), the fill
 // pass writes no lists, so no work items are published either: the insertion then reads no list
 // entry.  Bound by the latency of its few dependent loads and barriers.
+template<bool MERGE>
 __global__ void __launch_bounds__(1024) plan_kernel(int nBricks, BinBuffers b, ItemSplit split, bool first)
 {
   __shared__ int longest;
@@ -392,19 +396,36 @@ __global__ void __launch_bounds__(1024) plan_kernel(int nBricks, BinBuffers b, I
     }
     itemCap = int(min((long long)split.cap, cap));
   }
-  // pass 2: first items, in `order`
   const int perb = (nBricks + T - 1) / T, b0 = min(nBricks, tid * perb), b1 = min(nBricks, b0 + perb);
+  auto length = [&](int bb) { return b.offsets[3 * bb + 3] - b.offsets[3 * bb]; };
+  // Kahan: the bricks to be cut, in `order`, get their entry of the sums; without one, no cut
+  if (MERGE) {
+    auto cut = [&](int bb) { return itemCap < split.cap && length(bb) > itemCap; };
+    s = 0;
+    for (int k = b0; k < b1; ++k) s += cut(b.order[k]);
+    long long cuts = 0;
+    run = block_scan(s, cuts);
+    for (int k = b0; k < b1; ++k) {
+      const int bb = b.order[k];
+      const bool c = cut(bb);
+      b.merge.slot[bb] = c && run < b.merge.slots ? int(run) : -1;
+      b.merge.left[bb] = (length(bb) + itemCap - 1) / itemCap;
+      run += c;
+    }
+  }
+  // pass 2: first items, in `order` (a thread reads the slots it wrote)
+  auto items_of = [&](int bb) {
+    const int cap = MERGE && b.merge.slot[bb] < 0 ? split.cap : itemCap;
+    return (length(bb) + cap - 1) / cap;
+  };
   long long items = 0;
   s = 0;
-  for (int k = b0; k < b1; ++k) {
-    const int bb = b.order[k];
-    s += (b.offsets[3 * bb + 3] - b.offsets[3 * bb] + itemCap - 1) / itemCap;
-  }
+  for (int k = b0; k < b1; ++k) s += items_of(b.order[k]);
   run = block_scan(s, items);
   for (int k = b0; k < b1; ++k) {
     const int bb = b.order[k];
     b.itemStart[bb] = int(min(run, (long long)b.itemsCap));
-    run += (b.offsets[3 * bb + 3] - b.offsets[3 * bb] + itemCap - 1) / itemCap;
+    run += items_of(bb);
   }
   const bool fits = total <= b.listCap && items <= b.itemsCap;
   const bool ok = fits && prior == 0;
@@ -461,6 +482,12 @@ cudaError_t launch_traverse_spaces(const float *rot, int64_t n, uint32_t imgX, u
   return cudaGetLastError();
 }
 
+static void launch_plan(int nBricks, const BinBuffers &b, const ItemSplit &split, bool first, cudaStream_t st)
+{
+  if (b.merge.slot) plan_kernel<true><<<1, 1024, 0, st>>>(nBricks, b, split, first);
+  else plan_kernel<false><<<1, 1024, 0, st>>>(nBricks, b, split, first);
+}
+
 cudaError_t launch_batch_binning(const JobDesc *jobs, int nJobs, int totalSpaces, int totalBricks,
   int totalGroups, bool fast, float radius, const BinBuffers &b, const ItemSplit &split, cudaStream_t st)
 {
@@ -469,9 +496,9 @@ cudaError_t launch_batch_binning(const JobDesc *jobs, int nJobs, int totalSpaces
   if (totalSpaces > 0)
     batch_prep_kernel<<<(totalSpaces + 63) / 64, 64, 0, st>>>(jobs, nJobs, totalSpaces, hw, xmin, radius,
       b.prep, b.rec, b.status);
-  batch_bin_kernel<false><<<totalGroups, 256, 0, st>>>(jobs, nJobs, b.prep, b);
-  plan_kernel<<<1, 1024, 0, st>>>(totalBricks, b, split, true);
-  batch_bin_kernel<true><<<totalGroups, 256, 0, st>>>(jobs, nJobs, b.prep, b);
+  batch_bin_kernel<false><<<totalGroups, 256, 0, st>>>(jobs, nJobs, b.prep, b, split.cap);
+  launch_plan(totalBricks, b, split, true, st);
+  batch_bin_kernel<true><<<totalGroups, 256, 0, st>>>(jobs, nJobs, b.prep, b, split.cap);
   return cudaGetLastError();
 }
 
@@ -598,9 +625,9 @@ cudaError_t launch_binning(const BinGeom &g, const fr_traverse_space *spaces, in
   space_prep_kernel<<<(n + 63) / 64, 64, 0, st>>>(spaces, n, hw, xmin, radius, g.cx, g.cy, g.cz, nProj, b.prep, b.rec,
     b.status);
   const int blocks = bin_groups(g.nbx, g.nby, g.nbz);
-  bin_kernel<false><<<blocks, 256, 0, st>>>(g, b.prep, n, b);
-  plan_kernel<<<1, 1024, 0, st>>>(g.n_bricks, b, split, first);
-  bin_kernel<true><<<blocks, 256, 0, st>>>(g, b.prep, n, b);
+  bin_kernel<false><<<blocks, 256, 0, st>>>(g, b.prep, n, b, split.cap);
+  launch_plan(g.n_bricks, b, split, first, st);
+  bin_kernel<true><<<blocks, 256, 0, st>>>(g, b.prep, n, b, split.cap);
   return cudaGetLastError();
 }
 
@@ -645,8 +672,12 @@ void set_misc(BinBuffers &b, int *misc)
 // 0.51 ms, box 256 x 1,537 in two calls 4.17 -> 3.70 ms.  Two, eight and sixteen items per group
 // ran 556, 507 and 534 us at box 96 and 3.70, 3.75 and 3.81 ms at box 256.  From about 900,000
 // entries (1,400 box-256 projections) on, the capacity of 512 is the shorter one.
-// Kahan accumulators: an item's sums reach the volume by plain adds, so a brick is cut into
-// eight items at most (besides those of the capacity), which keeps them at FP32's last bits.
+// Kahan accumulators: the items of a cut brick are summed in FP64 (MergeBuffers) and reach the
+// volume as one add, as they did uncut.  Plain adds of up to eight items took the error against FP64
+// sums from 1.80e-7 to 1.92e-7 (box 32 x 64) and over eight calls from 1.09e-7 to 1.65e-7 (box 32 x
+// 400) and 3.7e-8 to 9.9e-8 (the same, nearest pixel); merged it is the uncut one's.  Box 32 x 64: 203 us
+// uncut, 57 cut with plain adds, 67 merged; box 64 x 1,500 1,794, 516 and 526.  Eight items a brick
+// at most.
 ItemSplit item_split(int itemCapacity, int brickGroups, const InsertConfig &cfg)
 {
   const int perGroup = cfg.fast ? kFastItemsPerGroup : kItemsPerGroup;

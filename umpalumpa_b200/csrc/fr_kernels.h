@@ -23,6 +23,15 @@ struct BinGeom {
 };
 
 // Scratch of one binning + insertion chunk.
+// Kahan accumulation: the items of a brick that is cut for idle groups are summed in FP64 before
+// the volume sees them, so that the cut leaves the sums as accurate as one item's (MergeBuffers.sums).
+struct MergeBuffers {
+  int *slot;     // [n_bricks] the brick's entry of `sums`, -1: not cut (nullptr: nothing is merged)
+  int *left;     // [n_bricks] items of the brick still to come
+  double *sums;  // [slots][3][kBrickVox] re, im, weight; zero between launches
+  int slots;
+};
+
 struct BinBuffers {
   SpacePrep *prep;        // [chunk capacity]
   SpaceRec *rec;          // [chunk capacity]
@@ -36,6 +45,7 @@ struct BinBuffers {
   int *status;            // [1] sticky FR_E_* of device-side failures
   int *workCounter;       // [1] next work item of the insertion
   int *itemCap;           // [1] list entries per work item
+  MergeBuffers merge;
   unsigned long long *stats;  // [4] pairs, items, chunks of the call
   int64_t listCap;
   int64_t itemsCap;
@@ -43,8 +53,8 @@ struct BinBuffers {
 
 // How the plan cuts the binned lists into work items: at most `cap` list entries per item and,
 // where `want` > 0, so few that the launch's brick groups get about `want` items between them,
-// but at least `least` entries, and (`perBrick` > 0) no brick is cut into more than `perBrick`
-// items for it.
+// but at least `least` entries, and (`perBrick` > 0: Kahan accumulation) no brick is cut into more
+// than `perBrick` items for it, and none without an entry of MergeBuffers.sums.
 struct ItemSplit {
   int cap;
   int want;
@@ -74,6 +84,7 @@ struct InsertParams {
   const WorkItem *items;
   const int *nItems;
   int *workCounter;
+  MergeBuffers merge;
   const float *table;  // lookup: the blob table; dynamic: the Kaiser (value, slope) table
   int tableElems;      // entries (float2 entries for the Kaiser table)
   float tableScale;    // Kaiser table: nodes per unit of d^2, (N - 1) / r^2
@@ -153,6 +164,13 @@ cudaError_t launch_batch_band(const JobDesc *jobs, int nJobs, int64_t totalUnits
 constexpr int kMiscStatus = 1, kMiscStats = 4;  // word indices: status; stats (4 x 64 bits)
 constexpr size_t kMiscBytes = 48;
 void set_misc(BinBuffers &b, int *misc);
+// Brick sums a Kahan call of this split can need (fewer than `want` bricks are longer than the
+// total / want entries of an item), and their bytes.
+inline int merge_slots(const ItemSplit &split, int64_t nBricks)
+{
+  return split.perBrick > 0 ? int(nBricks < split.want ? nBricks : split.want) : 0;
+}
+constexpr size_t kMergeSlotBytes = size_t(3) * 16 * 16 * 16 * sizeof(double);
 // Sets the carve-out preference of the kernels that run beside one another (fr_create).
 void prefer_shared_carveout();
 

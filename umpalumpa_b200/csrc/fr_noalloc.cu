@@ -186,13 +186,13 @@ extern "C" int fr_insert_noalloc(int device, void *stream, const fr_dims *d, con
   const size_t oItems = off;
   off += align256(size_t(itemsCap) * frb::kWorkItemBytes);
   if (off > kScratchBytes) return fail(FR_E_UNSUPPORTED, "volume too large for the 32 MiB scratch");
-  // what is left of the array takes the items of a finer split (few spaces, idle brick groups)
+  // what is left of the array takes the items of a finer split (few spaces, idle brick groups) and
+  // the brick sums that Kahan accumulation cuts for
   const int64_t spareItems = int64_t((kScratchBytes - off) / frb::kWorkItemBytes);
-  itemsCap += spareItems;
 
   char *sb = static_cast<char *>(base);
   int *misc = reinterpret_cast<int *>(sb + oMisc);
-  frb::BinBuffers bb;
+  frb::BinBuffers bb{};
   bb.prep = reinterpret_cast<frb::SpacePrep *>(sb + oPrep);
   bb.rec = reinterpret_cast<frb::SpaceRec *>(sb + oRec);
   bb.counts = reinterpret_cast<int *>(sb + oCounts);
@@ -227,6 +227,19 @@ extern "C" int fr_insert_noalloc(int device, void *stream, const fr_dims *d, con
   if (occ < 1) return fail(FR_E_UNSUPPORTED, "insertion kernel does not fit on an SM");
   frb::ItemSplit split = frb::item_split(kItemCapacity, sms * occ * frb::insert_groups(cfg), cfg);
   split.want = int(std::min<int64_t>(split.want, spareItems));
+  bb.itemsCap += split.want;
+  off += align256(size_t(split.want) * frb::kWorkItemBytes);
+  const size_t brickBytes = align256(size_t(g.n_bricks) * sizeof(int));
+  if (split.perBrick > 0 && off + 2 * brickBytes < kScratchBytes) {
+    bb.merge.slot = reinterpret_cast<int *>(sb + off);
+    bb.merge.left = reinterpret_cast<int *>(sb + off + brickBytes);
+    off += 2 * brickBytes;
+    bb.merge.sums = reinterpret_cast<double *>(sb + off);
+    bb.merge.slots = int(std::min<int64_t>(frb::merge_slots(split, g.n_bricks), int64_t((kScratchBytes - off) / frb::kMergeSlotBytes)));
+    if (bb.merge.slots > 0) e = cudaMemsetAsync(bb.merge.sums, 0, size_t(bb.merge.slots) * frb::kMergeSlotBytes, st);
+  } else if (split.perBrick > 0) {
+    split.want = 0;
+  }
 
   frb::InsertParams P{};
   P.volume = volume;
@@ -239,6 +252,7 @@ extern "C" int fr_insert_noalloc(int device, void *stream, const fr_dims *d, con
   P.items = bb.items;
   P.nItems = bb.nItems;
   P.workCounter = bb.workCounter;
+  P.merge = bb.merge;
   P.table = kaiserTable ? kaiser : table;
   P.tableElems = kaiserTable ? frb::kKaiserTableElems
                              : int(s->interpolation == FR_INTERPOLATION_LOOKUP ? d->table_elems : 0);
