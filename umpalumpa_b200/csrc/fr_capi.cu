@@ -496,7 +496,7 @@ int fr_init(fr_handle *h, const fr_dims *d, const fr_settings *s)
   h->launch.brick = 16;
   size_t smem = frb::insert_smem_bytes(cfg, int(d->table_elems));
   int occ = 0;
-  FR_CUDA(cudaFuncSetAttribute(frb::insert_kernel_ptr(cfg), cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+  FR_CUDA(frb::allow_insert_smem(cfg));
   FR_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, frb::insert_kernel_ptr(cfg), 256 * frb::insert_groups(cfg), smem));
   if (occ < 1) return fail(FR_E_UNSUPPORTED, "insertion kernel does not fit on an SM");
   if (h->launch.ctas_per_sm <= 0 || h->launch.ctas_per_sm > occ) h->launch.ctas_per_sm = occ;
@@ -864,7 +864,7 @@ int fr_batch_init(fr_handle *h, const fr_batch_limits *lim, const fr_settings *s
   h->launch.brick = 16;
   const size_t smem = frb::insert_smem_bytes(cfg, int(lim->table_elems));
   int occ = 0;
-  FR_CUDA(cudaFuncSetAttribute(frb::insert_kernel_ptr(cfg), cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+  FR_CUDA(frb::allow_insert_smem(cfg));
   FR_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, frb::insert_kernel_ptr(cfg), 256 * frb::insert_groups(cfg), smem));
   if (occ < 1) return fail(FR_E_UNSUPPORTED, "insertion kernel does not fit on an SM");
   if (h->launch.ctas_per_sm <= 0 || h->launch.ctas_per_sm > occ) h->launch.ctas_per_sm = occ;

@@ -692,9 +692,10 @@ int insert_groups(const InsertConfig &cfg)
   return cfg.groups > 0 && cfg.groups < mx ? cfg.groups : mx;
 }
 
-// Static shared memory of the insertion kernel (at most): the voxel lists of its 24 warps and a
-// few words.
-constexpr size_t kInsertStaticSmem = 12 << 10;
+// Shared memory a block may have, and what the insertion kernel takes of it statically (at most):
+// the voxel lists of its 24 warps (nearest pixel: none) and a few words.
+constexpr size_t kBlockSmem = 227 << 10;
+static size_t insert_static_smem(const InsertConfig &cfg) { return cfg.fast ? 1 << 10 : 12 << 10; }
 
 // Bytes of the kernel's table (the lookup table's entries, or the fixed Kaiser table of
 // dynamic interpolation); 0 when the mode reads none.
@@ -710,7 +711,7 @@ bool insert_lut_in_smem(const InsertConfig &cfg, int tableElems)
 {
   const size_t acc = size_t(insert_groups(cfg)) * size_t(cfg.kahan ? 18 : 12) * kBrickVox;
   const size_t t = table_bytes(cfg, tableElems);
-  return t > 0 && acc + t + kInsertStaticSmem <= (227u << 10);
+  return t > 0 && acc + t + insert_static_smem(cfg) <= kBlockSmem;
 }
 
 size_t insert_smem_bytes(const InsertConfig &cfg, int tableElems)
@@ -747,11 +748,20 @@ const void *insert_kernel_ptr(const InsertConfig &cfg)
   return reinterpret_cast<const void *>(pick_kernel(cfg));
 }
 
+// The limit belongs to the kernel on the device, not to a handle or launch: it is only ever set to
+// this one value, so that threads launching the kernel with other tables or group counts do not
+// lower it under one another.
+cudaError_t allow_insert_smem(const InsertConfig &cfg)
+{
+  return cudaFuncSetAttribute(pick_kernel(cfg), cudaFuncAttributeMaxDynamicSharedMemorySize,
+    int(kBlockSmem - insert_static_smem(cfg)));
+}
+
 cudaError_t launch_insert(const InsertParams &P, const InsertConfig &cfg, int grid, cudaStream_t st)
 {
   const size_t smem = insert_smem_bytes(cfg, P.tableElems);
   InsertFn k = pick_kernel(cfg);
-  cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+  const cudaError_t e = allow_insert_smem(cfg);
   if (e != cudaSuccess) return e;
   k<<<grid, kThreads * insert_groups(cfg), smem, st>>>(P);
   return cudaGetLastError();

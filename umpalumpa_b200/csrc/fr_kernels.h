@@ -186,6 +186,7 @@ cudaError_t launch_batch_binning(const JobDesc *jobs, int nJobs, int totalSpaces
   int totalGroups, bool fast, float radius, const BinBuffers &b, const ItemSplit &split, cudaStream_t st);
 cudaError_t launch_insert(const InsertParams &P, const InsertConfig &cfg, int grid, cudaStream_t st);
 size_t insert_smem_bytes(const InsertConfig &cfg, int tableElems);
+cudaError_t allow_insert_smem(const InsertConfig &cfg);  // lets the kernel be launched with as much
 int insert_groups(const InsertConfig &cfg);      // 256-thread groups per insertion CTA
 int insert_max_groups(const InsertConfig &cfg);  // the most groups a CTA of this variant holds
 // Whether the kernel's table goes to shared memory beside the launch's brick accumulators (a

@@ -216,7 +216,7 @@ extern "C" int fr_insert_noalloc(int device, void *stream, const fr_dims *d, con
 
   const size_t smem = frb::insert_smem_bytes(cfg, int(d->table_elems));
   int occ = 0, sms = 0;
-  if (e == cudaSuccess) e = cudaFuncSetAttribute(frb::insert_kernel_ptr(cfg), cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+  if (e == cudaSuccess) e = frb::allow_insert_smem(cfg);
   if (e == cudaSuccess)
     e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, frb::insert_kernel_ptr(cfg), 256 * frb::insert_groups(cfg), smem);
   if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);

@@ -174,7 +174,7 @@ std::vector<Candidate> candidates(fr_handle *h, Candidate *def)
     const size_t smem = frb::insert_smem_bytes(cfg, tableElems);
     const void *k = frb::insert_kernel_ptr(cfg);
     int occ = 0;
-    if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)) != cudaSuccess
+    if (frb::allow_insert_smem(cfg) != cudaSuccess
         || cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k, 256 * g, smem) != cudaSuccess) {
       cudaGetLastError();
       continue;
