@@ -281,7 +281,8 @@ typedef struct fr_launch_params {
 
 int fr_get_launch_params(const fr_handle *h, fr_launch_params *out);
 /* Overrides the launch parameters (0 keeps a field) and re-sizes the handle's scratch;
- * takes effect at the next fr_execute / fr_batch_execute. */
+ * takes effect at the next fr_execute / fr_batch_execute.  What is set stays set when the handle is
+ * initialised again; the other fields are then picked anew for the new strategy. */
 int fr_set_launch_params(fr_handle *h, const fr_launch_params *p);
 
 /* Per-call statistics of the last fr_execute, read after fr_synchronize: number of

@@ -216,14 +216,14 @@ static void set_kaiser(fr_handle *h)
   std::copy(std::begin(c), std::end(c), h->kaiser.begin());
 }
 
-// Under FR_TUNING_CACHED / ON_EXECUTE, takes the launch parameters of an equal strategy's
-// tuning file (fr_init / fr_batch_init, after the dims or limits and settings are set).
-static void apply_tuning_file(fr_handle *h)
+// The launch parameters an Init starts from (after the dims or limits and settings are set): the
+// caller's, not those another strategy resolved to, under those tuned for this strategy.
+static void resolve_launch(fr_handle *h)
 {
+  h->launch = h->held ? *h->held : h->want;
   h->tuned = false;
-  if (h->tuning == FR_TUNING_OFF || h->tuning_active) return;
   fr_launch_params p{};
-  if (!frb::tune_lookup(h, &p)) return;
+  if (h->tuning_active || !frb::tune_lookup(h, &p)) return;
   h->launch.item_capacity = p.item_capacity;
   h->launch.ctas_per_sm = p.ctas_per_sm;
   h->launch.groups = p.groups;
@@ -488,7 +488,7 @@ int fr_init(fr_handle *h, const fr_dims *d, const fr_settings *s)
   cfg.kahan = s->accumulation == FR_ACCUM_KAHAN;
   cfg.jobs = false;
   cfg.banded = s->layout != FR_LAYOUT_ROWS;  // fr_execute settles it per call
-  apply_tuning_file(h);
+  resolve_launch(h);
   cfg.groups = h->launch.groups;
   h->launch.groups = frb::insert_groups(cfg);
 
@@ -578,7 +578,7 @@ uint64_t fr_used_bytes(const fr_handle *h)
 int fr_get_launch_params(const fr_handle *h, fr_launch_params *out)
 {
   if (!h || !out) return fail(FR_E_INVALID, "NULL argument");
-  *out = h->launch;
+  *out = h->initialized ? h->launch : h->want;
   return FR_OK;
 }
 
@@ -587,20 +587,16 @@ int fr_set_launch_params(fr_handle *h, const fr_launch_params *p)
   if (!h || !p) return fail(FR_E_INVALID, "NULL argument");
   if (p->item_capacity < 0 || p->ctas_per_sm < 0 || p->groups < 0) return fail(FR_E_INVALID, "negative launch parameter");
   if (p->item_capacity > (1 << 20)) return fail(FR_E_UNSUPPORTED, "item_capacity above 2^20");
-  if (p->item_capacity > 0) h->launch.item_capacity = p->item_capacity;
-  if (p->ctas_per_sm > 0) h->launch.ctas_per_sm = p->ctas_per_sm;
-  if (p->groups > 0) h->launch.groups = p->groups;
-  if (h->initialized) {
-    // re-size the scratch so the item buffer and grid follow the new parameters
-    fr_settings s = h->settings;
-    if (h->batch) {
-      fr_batch_limits lim = h->blim;
-      return fr_batch_init(h, &lim, &s);
-    }
-    fr_dims d = h->dims;
-    return fr_init(h, &d, &s);
-  }
-  return FR_OK;
+  fr_launch_params held = h->launch;  // the other fields of this strategy stay
+  const auto set = [p](fr_launch_params &q) {
+    if (p->item_capacity > 0) q.item_capacity = p->item_capacity;
+    if (p->ctas_per_sm > 0) q.ctas_per_sm = p->ctas_per_sm;
+    if (p->groups > 0) q.groups = p->groups;
+  };
+  set(h->want);
+  set(held);
+  set(h->best);
+  return h->initialized ? frb::reinit(h, &held) : FR_OK;
 }
 
 int fr_get_exec_stats(const fr_handle *h, fr_exec_stats *out)
@@ -857,7 +853,7 @@ int fr_batch_init(fr_handle *h, const fr_batch_limits *lim, const fr_settings *s
   fill_config(cfg, *s);
   cfg.jobs = true;
   cfg.banded = true;  // batches insert from banded copies
-  apply_tuning_file(h);
+  resolve_launch(h);
   cfg.groups = h->launch.groups;
   h->launch.groups = frb::insert_groups(cfg);
   if (h->launch.item_capacity <= 0) h->launch.item_capacity = frb::kItemCapacity;
@@ -1217,3 +1213,19 @@ int fr_compute_traverse_spaces_sym(const float *rotations, uint64_t n, const flo
 }
 
 }// extern "C"
+
+int frb::reinit(fr_handle *h, const fr_launch_params *held)
+{
+  const fr_settings s = h->settings;
+  h->held = held;
+  int rc;
+  if (h->batch) {
+    const fr_batch_limits lim = h->blim;
+    rc = fr_batch_init(h, &lim, &s);
+  } else {
+    const fr_dims d = h->dims;
+    rc = fr_init(h, &d, &s);
+  }
+  h->held = nullptr;
+  return rc;
+}

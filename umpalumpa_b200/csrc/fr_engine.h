@@ -10,8 +10,13 @@ namespace frb {
 // finished batched launch; valid once that launch's work has completed on the stream.
 int batch_device_status(const fr_handle *h);
 
-// Autotuner hooks (fr_tune.cu).  tune_lookup: the launch parameters of the tuning file of the
-// handle's current strategy (dims/limits and settings set), if the file exists.  tune_single:
+// Initialises the handle again for the same strategy, from `held` in place of the caller's launch
+// parameters (nullptr: from those), so that the item buffer and grid follow.
+int reinit(fr_handle *h, const fr_launch_params *held);
+
+// Autotuner hooks (fr_tune.cu).  tune_lookup: the launch parameters the handle's last search found
+// for its current strategy (dims/limits and settings set), else, unless the approach is
+// FR_TUNING_OFF, those of the strategy's tuning file, if it exists.  tune_single:
 // the search of fr_autotune, run by fr_execute under FR_TUNING_ON_EXECUTE.
 bool tune_lookup(const fr_handle *h, fr_launch_params *out);
 int tune_single(fr_handle *h, const void *fft, const float *scales, uint64_t nProj,

@@ -37,7 +37,9 @@ struct fr_handle {
   std::array<float2, frb::kKaiserDegree + 1> kaiser{};  // dynamic blob, alpha <= 15 (kaiser_polynomial)
   frb::BinGeom geom{};
   frb::InsertConfig cfg{};
-  fr_launch_params launch{};
+  fr_launch_params want{};                      // launch parameters as set by the caller (0: default)
+  fr_launch_params launch{};                    // those of the current Init, resolved from `want`
+  const fr_launch_params *held = nullptr;       // in their place during a re-initialisation (reinit)
   int64_t chunk_cap = 0;
   int grid = 0;
   void *scratch = nullptr;
@@ -89,6 +91,8 @@ struct fr_handle {
   std::string device_name;
   int tuning = FR_TUNING_OFF;
   std::string tuning_dir;      // empty: the default directory
+  fr_launch_params best{};     // of the handle's last search, for the strategy best_key
+  std::string best_key;
   bool tuned = false;          // this Init's parameters came from a tuning file or a search
   bool tuning_active = false;  // a search is running: no tuning-file lookups, no nested search
 };

@@ -201,7 +201,6 @@ int search(fr_handle *h, Run run, Sync sync, uint32_t sample, fr_tune_report *re
     if (e0) cudaEventDestroy(e0);
     return fail(FR_E_CUDA, "cudaEventCreate failed");
   }
-  const fr_launch_params saved = h->launch;
   h->tuning_active = true;
   double best = std::numeric_limits<double>::infinity(), defMs = -1.0;
   Candidate bestC = def;
@@ -212,7 +211,7 @@ int search(fr_handle *h, Run run, Sync sync, uint32_t sample, fr_tune_report *re
     p.item_capacity = c.item;
     p.ctas_per_sm = c.ctas;
     p.groups = c.groups;
-    if ((rc = fr_set_launch_params(h, &p)) != FR_OK) break;  // re-sizing failed: stop
+    if ((rc = frb::reinit(h, &p)) != FR_OK) break;  // re-sizing failed: stop
     if (h->launch.ctas_per_sm != c.ctas || h->launch.groups != c.groups) continue;  // clamped: a duplicate
     if (run() != FR_OK || sync() != FR_OK) continue;  // warm-up; a failing shape is skipped
     float ms = std::numeric_limits<float>::infinity();
@@ -240,8 +239,8 @@ int search(fr_handle *h, Run run, Sync sync, uint32_t sample, fr_tune_report *re
   if (rc == FR_OK && trials == 0) rc = fail(FR_E_CUDA, "no launch shape ran the tuning sample");
   if (rc != FR_OK) {
     const std::string msg = fr_last_error();
-    fr_set_launch_params(h, &saved);
     h->tuning_active = false;
+    frb::reinit(h, nullptr);
     return fail(rc, "autotuning failed: " + msg);
   }
   if (defMs > 0 && best > kKeepDefault * defMs) {
@@ -252,11 +251,12 @@ int search(fr_handle *h, Run run, Sync sync, uint32_t sample, fr_tune_report *re
   p.item_capacity = bestC.item;
   p.ctas_per_sm = bestC.ctas;
   p.groups = bestC.groups;
-  rc = fr_set_launch_params(h, &p);
   h->tuning_active = false;
-  if (rc) return rc;
-  h->tuned = true;
   const std::string key = strategy_key(h);
+  h->best = p;
+  h->best_key = key;
+  rc = frb::reinit(h, nullptr);
+  if (rc) return rc;
   if (h->tuning != FR_TUNING_OFF) write_tuning_file(tuning_path(h, key), key, h->launch, best, defMs);
   if (rep) {
     std::memset(rep, 0, sizeof(*rep));
@@ -275,7 +275,11 @@ int search(fr_handle *h, Run run, Sync sync, uint32_t sample, fr_tune_report *re
 bool frb::tune_lookup(const fr_handle *h, fr_launch_params *out)
 {
   const std::string key = strategy_key(h);
-  return read_tuning_file(tuning_path(h, key), key, out);
+  if (h->best_key == key) {
+    *out = h->best;
+    return true;
+  }
+  return h->tuning != FR_TUNING_OFF && read_tuning_file(tuning_path(h, key), key, out);
 }
 
 int frb::tune_single(fr_handle *h, const void *fft, const float *scales, uint64_t nProj,
@@ -312,7 +316,11 @@ int fr_set_tuning(fr_handle *h, int approach, const char *directory)
   h->tuned = false;
   if (h->initialized && approach != FR_TUNING_OFF) {
     fr_launch_params p{};
-    if (frb::tune_lookup(h, &p)) return fr_set_launch_params(h, &p);  // re-init marks it tuned
+    const std::string key = strategy_key(h);
+    if (read_tuning_file(tuning_path(h, key), key, &p)) {
+      h->best_key.clear();
+      return frb::reinit(h, nullptr);  // takes the file and marks the handle tuned
+    }
   }
   return FR_OK;
 }
