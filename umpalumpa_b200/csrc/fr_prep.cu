@@ -175,7 +175,7 @@ struct fr_prep {
 namespace {
 
 // Side of the fused route for these settings (0: cuFFT route).  It is the faster one at every side
-// and storage it covers (fr_prep_fft.cuh).
+// and storage it covers, few images or many (fr_prep_fft.cuh; kSplit has the one exception).
 int fused_side(const fr_prep_settings &s)
 {
   if (s.fft == FR_PREP_FFT_CUFFT || s.size_x != s.size_y) return 0;
@@ -200,14 +200,37 @@ template<class F> cudaError_t with_side(int n, F f)
   }
 }
 
-template<int N, int STORAGE, bool BANDED = false> cudaError_t launch_fused(fr_prep *p, const frb::prepfft::Args &a)
+template<int N, int STORAGE, bool BANDED, int SPLIT> cudaError_t launch_split(fr_prep *p, const frb::prepfft::Args &a)
 {
   using Sh = frb::prepfft::Shape<N>;
-  auto *kernel = frb::prepfft::prep_fft_kernel<N, STORAGE, BANDED>;
-  const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(Sh::smem));
+  constexpr size_t smem = frb::prepfft::kSmem<N, SPLIT>;
+  auto *kernel = frb::prepfft::prep_fft_kernel<N, STORAGE, BANDED, SPLIT>;
+  const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
   if (e != cudaSuccess) return e;
-  kernel<<<std::min(a.n, p->ctas), Sh::threads, Sh::smem, p->stream>>>(a);
-  return cudaGetLastError();
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(SPLIT > 1 ? a.n * SPLIT : std::min(a.n, p->ctas));
+  cfg.blockDim = dim3(Sh::threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = p->stream;
+  cudaLaunchAttribute cluster;
+  cluster.id = cudaLaunchAttributeClusterDimension;
+  cluster.val.clusterDim.x = SPLIT;
+  cluster.val.clusterDim.y = cluster.val.clusterDim.z = 1;
+  cfg.attrs = &cluster;
+  cfg.numAttrs = SPLIT > 1 ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, kernel, a);
+}
+
+// A call of as many images as the CTAs can take in clusters takes them so where it pays (kSplits);
+// their rows of S fit the scratch.
+template<int N, int STORAGE, bool BANDED = false> cudaError_t launch_fused(fr_prep *p, const frb::prepfft::Args &a)
+{
+  using namespace frb::prepfft;
+  if constexpr (kSplits<N, STORAGE>) {
+    static_assert(Shape<N>::l2Rows * kSplit >= N, "scratch for ctas / kSplit images");
+    if (a.n <= p->ctas / kSplit) return launch_split<N, STORAGE, BANDED, kSplit>(p, a);
+  }
+  return launch_split<N, STORAGE, BANDED, 1>(p, a);
 }
 
 }// namespace

@@ -224,11 +224,29 @@ template<int N> struct Shape {
   static constexpr bool ahead = N >= 256;
 };
 
+// CTAs an image is split between in a call of few images: FP32 sides 320 and 384, where one CTA per
+// image is slower than cuFFT up to 12 images.  It is the latency of the passes' N / 32 rounds,
+// which the CTAs of a cluster share: 1, 8, 32 and 37 images of side 320 take 19, 19, 21 and 33 us
+// (one CTA each 51; cuFFT 43, 48, 64 and 68), of side 384 21, 21, 23 and 41 (70; 56, 62, 86 and 88).
+// Elsewhere one CTA per image is no slower than cuFFT, but for side 256 up to 8 images (35 against 31).
+constexpr int kSplit = 4;
+template<int N, int STORAGE> constexpr bool kSplits = N > 256 && STORAGE == FR_STORAGE_FP32;
+
+template<int N, int SPLIT> constexpr int kNearRows = SPLIT > 1 ? 0 : Shape<N>::smemRows;
+template<int N, int SPLIT> constexpr size_t kSmem =
+  Shape<N>::smem - size_t(Shape<N>::smemRows - kNearRows<N, SPLIT>) * Shape<N>::pitch * sizeof(float2);
+
 // BANDED: FP32 output in bands (16-bit output takes its layout in the last pass).
-template<int N, int STORAGE, bool BANDED>
+// SPLIT > 1: clusters of SPLIT CTAs take one image each (gridDim.x = SPLIT n), all of S in L2, the
+// rounds of the passes dealt between the CTAs; the values are the same bit for bit.
+template<int N, int STORAGE, bool BANDED, int SPLIT>
 __global__ void __launch_bounds__(Shape<N>::threads, Shape<N>::ctas) prep_fft_kernel(Args a)
 {
+  static_assert(SPLIT == 1 || STORAGE == FR_STORAGE_FP32, "the CTAs of an image share no maximum");
   using Sh = Shape<N>;
+  constexpr int nearRows = kNearRows<N, SPLIT>;
+  const int group = int(blockIdx.x) / SPLIT, groups = int(gridDim.x) / SPLIT;
+  const int first = 16 * (int(blockIdx.x) % SPLIT);  // of the CTA's rounds, 16 columns or rows each
   constexpr int TT = Sh::TT, H = N / 2;
   extern __shared__ float2 sm[];
   float2 *tw = sm;            // [16][TT]
@@ -238,14 +256,14 @@ __global__ void __launch_bounds__(Shape<N>::threads, Shape<N>::ctas) prep_fft_ke
   __shared__ float red[Sh::threads / 32];
   const int tid = threadIdx.x;
   for (int i = tid; i < N; i += Sh::threads) tw[i] = a.tw[i];
-  float2 *far = a.scratch + size_t(blockIdx.x) * Sh::l2Rows * Sh::pitch;
+  float2 *far = a.scratch + size_t(group) * (N - nearRows) * Sh::pitch;
   auto S = [&](int row) -> float2 * {
-    return row < Sh::smemRows ? near + row * Sh::pitch : far + size_t(row - Sh::smemRows) * Sh::pitch;
+    return row < nearRows ? near + row * Sh::pitch : far + size_t(row - nearRows) * Sh::pitch;
   };
   const bool pairs = (reinterpret_cast<uintptr_t>(a.images) & 7) == 0;
   __syncthreads();
 
-  for (int img = blockIdx.x; img < a.n; img += gridDim.x) {
+  for (int img = group; img < a.n; img += groups) {
     const float *I = a.images + size_t(img) * N * N;
     // ---- 1. column pass, 16 column pairs at a time, the next ones' points in flight
     const int m = tid & 15, cj = tid >> 4;
@@ -261,15 +279,15 @@ __global__ void __launch_bounds__(Shape<N>::threads, Shape<N>::ctas) prep_fft_ke
           v[q] = make_float2(__ldcs(p + size_t(TT * q) * N), __ldcs(p + size_t(TT * q) * N + 1));
       }
     };
-    if (Sh::ahead && cj < TT) load_columns(0);
-    for (int m0 = 0; m0 < H; m0 += 16) {
+    if (Sh::ahead && cj < TT) load_columns(first);
+    for (int m0 = first; m0 < H; m0 += 16 * SPLIT) {
       if (cj < TT) {
         if (!Sh::ahead) load_columns(m0);
         dft<16>(v);
 #pragma unroll
         for (int k1 = 0; k1 < 16; ++k1)
           buf[(k1 * TT + cj) * 16 + m] = k1 ? cmul(v[k1], tw[k1 * TT + cj]) : v[0];
-        if (Sh::ahead && m0 + 16 < H) load_columns(m0 + 16);
+        if (Sh::ahead && m0 + 16 * SPLIT < H) load_columns(m0 + 16 * SPLIT);
       }
       __syncthreads();
       if (tid < 256) {
@@ -280,15 +298,18 @@ __global__ void __launch_bounds__(Shape<N>::threads, Shape<N>::ctas) prep_fft_ke
         dft<TT>(u);
 #pragma unroll
         for (int k2 = 0; k2 < TT; ++k2) {
-          if (16 * k2 < Sh::smemRows) near[(k1 + 16 * k2) * Sh::pitch + m0 + m] = u[k2];
-          else far[(k1 + 16 * k2 - Sh::smemRows) * Sh::pitch + m0 + m] = u[k2];
+          if (16 * k2 < nearRows) near[(k1 + 16 * k2) * Sh::pitch + m0 + m] = u[k2];
+          else far[(k1 + 16 * k2 - nearRows) * Sh::pitch + m0 + m] = u[k2];
         }
       }
       __syncthreads();
     }
+    // the cluster's column spectra, written to global memory, before any of its CTAs reads them
+    if (SPLIT > 1)
+      asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
     // the first columns of the CTA's next image, on their way to L2 during the row pass
-    if (img + int(gridDim.x) < a.n && tid < N)
-      asm volatile("prefetch.global.L2 [%0];" ::"l"(I + size_t(gridDim.x) * N * N + size_t(tid) * N));
+    if (img + groups < a.n && tid < N)
+      asm volatile("prefetch.global.L2 [%0];" ::"l"(I + size_t(groups) * N * N + size_t(tid) * N));
     // ---- 2. row pass, 16 rows ky (with their mirrors N - ky) at a time
     float amax = 0.f;
     // The processed value F[origY][x] (twice: the separations leave their halves out) of output
@@ -322,7 +343,7 @@ __global__ void __launch_bounds__(Shape<N>::threads, Shape<N>::ctas) prep_fft_ke
       }
     };
     const int half = a.outY / 2;  // rows 0..half and N - (half - 1)..N - 1 are wanted
-    for (int r0 = 0; r0 < H && r0 <= half; r0 += 16) {
+    for (int r0 = first; r0 < H && r0 <= half; r0 += 16 * SPLIT) {
       {
         const int r = tid / TT, j = tid - r * TT, ky = r0 + r;
         if (r < 16) {
