@@ -851,6 +851,7 @@ int fr_batch_init(fr_handle *h, const fr_batch_limits *lim, const fr_settings *s
   fill_config(cfg, *s);
   cfg.jobs = true;
   cfg.banded = true;  // batches insert from banded copies
+  h->batch = true;    // the strategy's key is a batch's
   resolve_launch(h);
   cfg.groups = h->launch.groups;
   h->launch.groups = frb::insert_groups(cfg);
@@ -920,7 +921,6 @@ int fr_batch_init(fr_handle *h, const fr_batch_limits *lim, const fr_settings *s
       h->stream));
   }
   FR_CUDA(cudaStreamSynchronize(h->stream));
-  h->batch = true;
   h->initialized = true;
   return FR_OK;
 }
