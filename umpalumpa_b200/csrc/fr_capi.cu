@@ -217,10 +217,12 @@ static void set_kaiser(fr_handle *h)
 }
 
 // The launch parameters an Init starts from (after the dims or limits and settings are set): the
-// caller's, not those another strategy resolved to, under those tuned for this strategy.
+// caller's, not those another strategy resolved to, under those tuned for this strategy.  A
+// re-initialisation that brings its own (reinit) takes those, of a strategy as tuned as before.
 static void resolve_launch(fr_handle *h)
 {
   h->launch = h->held ? *h->held : h->want;
+  if (h->held) return;
   h->tuned = false;
   fr_launch_params p{};
   if (h->tuning_active || !frb::tune_lookup(h, &p)) return;
