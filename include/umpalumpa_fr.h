@@ -270,8 +270,8 @@ int fr_band_projections(const void *fft, uint64_t n, uint64_t fft_x, uint64_t ff
  * groups per CTA (the thread-block shape; each group accumulates one brick in shared memory,
  * the groups of a CTA share one copy of the blob table).  These are what the reference's KTT
  * search varies for FRCUDA (BLOCK_DIM, TILE, GRID_DIM_Z, fr_cuda.cpp:100-157).  The default
- * capacity, 512, is an upper bound: a call whose lists would leave brick groups idle is cut into
- * shorter items.  Any other capacity is taken as given. */
+ * capacity, 512, and one the autotuner picked are upper bounds: a call whose lists would leave brick
+ * groups idle is cut into shorter items.  Any other capacity that the caller sets is taken as given. */
 typedef struct fr_launch_params {
   int32_t brick;
   int32_t item_capacity;

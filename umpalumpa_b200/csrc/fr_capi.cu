@@ -232,10 +232,13 @@ static void resolve_launch(fr_handle *h)
   h->tuned = true;
 }
 
-// The item split of the handle's launch shape (after its grid and groups are settled).
+// The item split of the handle's launch shape (after its grid and groups are settled).  A capacity
+// that is the caller's is taken as given, the default and a tuned one are upper bounds.
 static frb::ItemSplit handle_split(const fr_handle *h)
 {
-  return frb::item_split(h->launch.item_capacity, h->grid * frb::insert_groups(h->cfg), h->cfg);
+  const int cap = h->launch.item_capacity;
+  const bool given = cap == h->want.item_capacity && cap != frb::kItemCapacity;
+  return frb::item_split(cap, given ? 0 : h->grid * frb::insert_groups(h->cfg), h->cfg);
 }
 
 // The Kahan handle's brick sums, for its split and at most nBricks bricks.  Where their memory

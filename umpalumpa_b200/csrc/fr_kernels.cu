@@ -681,7 +681,7 @@ void set_misc(BinBuffers &b, int *misc)
 ItemSplit item_split(int itemCapacity, int brickGroups, const InsertConfig &cfg)
 {
   const int perGroup = cfg.fast ? kFastItemsPerGroup : kItemsPerGroup;
-  return { itemCapacity, itemCapacity == kItemCapacity ? perGroup * brickGroups : 0, cfg.fast ? 32 : 2, cfg.kahan ? 8 : 0 };
+  return { itemCapacity, perGroup * brickGroups, cfg.fast ? 32 : 2, cfg.kahan ? 8 : 0 };
 }
 
 int insert_max_groups(const InsertConfig &cfg) { return (cfg.kahan ? 2 : 3) + (cfg.fast ? 1 : 0); }

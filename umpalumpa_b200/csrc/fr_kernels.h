@@ -62,12 +62,10 @@ struct ItemSplit {
   int perBrick;
 };
 
-// The default item capacity; only with it does the plan shorten items (`want` > 0), any other
-// capacity (fr_set_launch_params, the autotuner) is taken as given.
+// The default item capacity.
 constexpr int kItemCapacity = 512;
 constexpr int kItemsPerGroup = 4;
 constexpr int kFastItemsPerGroup = 1;  // nearest pixel: an entry costs a tenth of a blob entry
-
 
 // Degree of the dynamic blob's polynomial (alpha <= 15).
 constexpr int kKaiserDegree = 12;
@@ -115,6 +113,7 @@ struct InsertConfig {
   bool banded;  // half-planes in 4-row bands (always for a batch); else row-major
 };
 
+// The split of a launch of `brickGroups` groups (0: the capacity as given).
 ItemSplit item_split(int itemCapacity, int brickGroups, const InsertConfig &cfg);
 
 using InsertFn = void (*)(InsertParams);
