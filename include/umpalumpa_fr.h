@@ -351,8 +351,9 @@ int fr_batch_execute(fr_handle *h, const fr_job *jobs, uint64_t n_jobs, const fl
  * every equal strategy (strategy_manager.cpp:14-83, ktt_strategy_base.hpp:110-134).  Here the
  * search is over fr_launch_params -- groups per CTA x CTAs per SM x traverse spaces per work
  * item, every combination that fits on an SM -- each timed with CUDA events on the handle's
- * stream, and the best is stored in a tuning file named by the strategy key: device name and SM
- * count, payload sizes (for a batch: its limits), settings, and the size class of the job. */
+ * stream, and the best is stored in a tuning file named by the strategy key: kernel revision,
+ * device name and SM count, payload sizes (for a batch: its limits), settings, and the size class
+ * of the job. */
 enum {
   FR_TUNING_OFF = 0,        /* defaults, no tuning files (the default)                        */
   FR_TUNING_CACHED = 1,     /* fr_init / fr_batch_init use the tuning file of an equal strategy */

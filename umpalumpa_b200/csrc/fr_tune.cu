@@ -60,6 +60,10 @@ int size_class(uint64_t n)  // ceil(log2 n): jobs of one class share a tuning fi
   return c;
 }
 
+// Raised whenever a change of the insertion kernels or of the item split moves the best launch shape:
+// files of another revision are not taken.
+constexpr int kKernelRevision = 2;
+
 std::string strategy_key(const fr_handle *h)
 {
   std::string dev = h->device_name;
@@ -70,16 +74,16 @@ std::string strategy_key(const fr_handle *h)
   if (h->batch) {
     const fr_batch_limits &l = h->blim;
     std::snprintf(buf, sizeof buf,
-      "fr-b200 device=%s sms=%d batch max_jobs=%llu max_spaces=%llu max_bricks=%llu max_side=%llu table=%llu",
-      dev.c_str(), h->num_sms, (unsigned long long)l.max_jobs, (unsigned long long)l.max_spaces,
+      "fr-b200 kernels=%d device=%s sms=%d batch max_jobs=%llu max_spaces=%llu max_bricks=%llu max_side=%llu table=%llu",
+      kKernelRevision, dev.c_str(), h->num_sms, (unsigned long long)l.max_jobs, (unsigned long long)l.max_spaces,
       (unsigned long long)l.max_bricks, (unsigned long long)l.max_volume_side, (unsigned long long)l.table_elems);
   } else {
     const fr_dims &d = h->dims;
     std::snprintf(buf, sizeof buf,
-      "fr-b200 device=%s sms=%d single fft=%llux%llu volume=%llux%llux%llu table=%llu spaces_class=%d", dev.c_str(),
-      h->num_sms, (unsigned long long)d.fft_x, (unsigned long long)d.fft_y, (unsigned long long)d.volume_x,
-      (unsigned long long)d.volume_y, (unsigned long long)d.volume_z, (unsigned long long)d.table_elems,
-      size_class(std::min<uint64_t>(d.n_spaces, 65536)));
+      "fr-b200 kernels=%d device=%s sms=%d single fft=%llux%llu volume=%llux%llux%llu table=%llu spaces_class=%d",
+      kKernelRevision, dev.c_str(), h->num_sms, (unsigned long long)d.fft_x, (unsigned long long)d.fft_y,
+      (unsigned long long)d.volume_x, (unsigned long long)d.volume_y, (unsigned long long)d.volume_z,
+      (unsigned long long)d.table_elems, size_class(std::min<uint64_t>(d.n_spaces, 65536)));
   }
   char set[256];
   std::snprintf(set, sizeof set,
