@@ -94,6 +94,12 @@ typedef struct fr_settings {
   int32_t layout;         /* FR_LAYOUT_*                                                      */
 } fr_settings;
 
+/* alpha is positive (the blob's Fourier value, and with it every dynamic weight, is NaN for
+ * others).  Below 4 the weight at the blob's edge is a sizeable part of its peak (0.8 at alpha 1), so
+ * that a pixel whose squared distance rounds to the other side of the radius' -- the engine's distance
+ * is fused, FRCPU's is not -- shows in its voxel: relative L2 against FRCPU up to 1e-4 on jobs of
+ * few projections, in place of 1e-6; every other voxel agrees as at alpha 15. */
+
 /* Fills the reference defaults (interpolation dynamic, order 0, type fast, alpha 15,
  * radius 1.9) plus max_resolution 0.5, FP32 storage, plain accumulation, layout auto. */
 void fr_settings_default(fr_settings *s);

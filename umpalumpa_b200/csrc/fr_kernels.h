@@ -129,7 +129,7 @@ InsertFn pick_insert_batch_bf16(const InsertConfig &cfg);
 InsertFn pick_insert_batch_fp16(const InsertConfig &cfg);
 
 // Coefficients, constant first, of the polynomial in u = 1 - d2 / r^2 that interpolates
-// ks I0(alpha sqrt(u)), |alpha| <= 15.
+// ks I0(alpha sqrt(u)), 0 < alpha <= 15 (cIw0, and so ks, is NaN for any other below).
 void kaiser_polynomial(float alpha, float ks, float2 (&c)[kKaiserDegree + 1]);
 // Dynamic interpolation's Kaiser (value, slope) table: kKaiserTableElems float2 entries.
 cudaError_t launch_kaiser_table(float *table, int order, float alpha, float radius, float iw0, cudaStream_t st);
