@@ -67,7 +67,7 @@ enum { FR_ACCUM_PLAIN = 0, FR_ACCUM_KAHAN = 1 };
  *                     insertion is 12 % faster, the whole call 7 %), or reads the rows in
  *                     place where that memory cannot be had, the call inserts fewer spaces
  *                     than a third of the payload's projections, or it is a nearest-pixel
- *                     insertion (kFast);
+ *                     insertion (kFast) of more than 8 MB of bands;
  *   FR_LAYOUT_ROWS:   reads the caller's rows in place (no copy, no extra memory);
  *   FR_LAYOUT_BANDED: the payload is already banded (fr_band_projections, or fr_prep with
  *                     out_layout FR_LAYOUT_BANDED); fr_execute reads it in place.

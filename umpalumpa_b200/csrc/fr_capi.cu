@@ -733,11 +733,13 @@ int fr_execute(fr_handle *h, const void *fft, const float *scales, uint64_t nPro
   // binning on the compute stream; the insertion waits for both.
   // A call that inserts few spaces of a large payload reads the rows in place: the copy (about
   // 0.1 us per box-256 projection) pays for itself from about one space per three projections.
-  // Nearest-pixel insertion reads one pixel per voxel, and the copy never pays (whole calls, rows against
-  // bands: box 16 x 20 47 / 50 us, 48 x 300 62 / 65, 128 x 60 56 / 57, 96 x 2,000 321 / 345, 256 x 4,000
-  // 1,681 / 1,946).
+  // Nearest-pixel insertion reads one pixel per voxel, so the bands save it little: it takes them
+  // only while the copy is small enough to stay in L2 and end beside the binning (rows against
+  // bands: box 48 x 300, 3 MB, 101 / 102 us; box 96 x 2,000, 75 MB, 321 / 345 us; box 256 x 4,000,
+  // 1,057 MB, 1,681 / 1,946 us).
   bool banded = s.layout == FR_LAYOUT_BANDED, bandCopy = false;
-  if (s.layout == FR_LAYOUT_AUTO && s.type != FR_TYPE_FAST && nSpaces * 3 >= nProj) {
+  const bool bandsPay = s.type != FR_TYPE_FAST || size_t(nProj) * bandPlaneBytes <= (size_t(8) << 20);
+  if (s.layout == FR_LAYOUT_AUTO && bandsPay && nSpaces * 3 >= nProj) {
     int rc = ensure_band(h, size_t(nProj) * bandPlaneBytes, true, bandCopy);
     if (rc) return rc;
     if (bandCopy) {
