@@ -486,7 +486,7 @@ int fr_init(fr_handle *h, const fr_dims *d, const fr_settings *s)
   set_kaiser(h);
   frb::InsertConfig &cfg = h->cfg;
   cfg.fast = s->type == FR_TYPE_FAST;
-  cfg.mode = s->interpolation == FR_INTERPOLATION_LOOKUP ? 0 : (s->alpha <= 15.f ? 1 : 3);
+  cfg.mode = s->interpolation == FR_INTERPOLATION_LOOKUP ? 0 : (s->alpha <= 15.f ? 1 : 2);
   int taps = int(std::floor(2.f * s->blob_radius)) + 1;
   cfg.taps = taps <= 4 ? 4 : 8;  // the kernel's blob window: 4x4 for r < 2, 8x8 for r < 4
   cfg.storage = s->storage;
@@ -545,7 +545,7 @@ int fr_init(fr_handle *h, const fr_dims *d, const fr_settings *s)
   const size_t oOrder = take(size_t(g.n_bricks) * sizeof(int));
   const size_t oItems = take(size_t(itemsCap) * frb::kWorkItemBytes);
   const size_t oMisc = take(64);
-  const size_t oKaiser = take(cfg.mode == 3 && !cfg.fast ? size_t(frb::kKaiserTableElems) * sizeof(float2) : 0);
+  const size_t oKaiser = take(cfg.mode == 2 && !cfg.fast ? size_t(frb::kKaiserTableElems) * sizeof(float2) : 0);
   FR_CUDA(cudaMalloc(&h->scratch, off));
   h->scratch_bytes = off;
   char *base = static_cast<char *>(h->scratch);
@@ -565,7 +565,7 @@ int fr_init(fr_handle *h, const fr_dims *d, const fr_settings *s)
   FR_CUDA(cudaMemcpyAsync(base + oOrder, order.data(), order.size() * sizeof(int), cudaMemcpyHostToDevice, h->stream));
   FR_CUDA(cudaMemsetAsync(misc, 0, 64, h->stream));
   h->kaiser_table = nullptr;
-  if (cfg.mode == 3 && !cfg.fast) {
+  if (cfg.mode == 2 && !cfg.fast) {
     h->kaiser_table = reinterpret_cast<float *>(base + oKaiser);
     FR_CUDA(frb::launch_kaiser_table(h->kaiser_table, s->blob_order, s->alpha, s->blob_radius, h->constants.cIw0,
       h->stream));
@@ -733,10 +733,10 @@ int fr_execute(fr_handle *h, const void *fft, const float *scales, uint64_t nPro
   // binning on the compute stream; the insertion waits for both.
   // A call that inserts few spaces of a large payload reads the rows in place: the copy (about
   // 0.1 us per box-256 projection) pays for itself from about one space per three projections.
-  // Nearest-pixel insertion reads one pixel per voxel, so the bands save it little: it takes them
-  // only while the copy is small enough to stay in L2 and end beside the binning (rows against
-  // bands: box 48 x 300, 3 MB, 101 / 102 us; box 96 x 2,000, 75 MB, 321 / 345 us; box 256 x 4,000,
-  // 1,057 MB, 1,681 / 1,946 us).
+  // Nearest-pixel insertion reads one pixel per voxel, so the bands save it little.  Up to 8 MB, where
+  // the copy stays in L2 and ends beside the binning, the layout's default copies there too; beyond,
+  // it would cost a tenth of the call (whole calls, rows against bands: box 16 x 20 47 / 50 us, box 48 x
+  // 300, 3 MB, 62 / 65; box 96 x 2,000, 75 MB, 321 / 345; box 256 x 4,000, 1,057 MB, 1,681 / 1,946).
   bool banded = s.layout == FR_LAYOUT_BANDED, bandCopy = false;
   const bool bandsPay = s.type != FR_TYPE_FAST || size_t(nProj) * bandPlaneBytes <= (size_t(8) << 20);
   if (s.layout == FR_LAYOUT_AUTO && bandsPay && nSpaces * 3 >= nProj) {
@@ -769,7 +769,6 @@ int fr_execute(fr_handle *h, const void *fft, const float *scales, uint64_t nPro
   P.lutInSmem = frb::insert_lut_in_smem(h->cfg, P.tableElems);
   P.genericTaps = int(h->dims.fft_x) < h->cfg.taps || int(h->dims.fft_y) < h->cfg.taps || P.tableElems > frb::kLutSmemMax;
   P.c = h->constants;
-  P.order = s.blob_order;
   P.nProj = int(nProj);
   P.fftX = int(h->dims.fft_x);
   P.fftY = int(h->dims.fft_y);
@@ -816,7 +815,7 @@ int fr_execute(fr_handle *h, const void *fft, const float *scales, uint64_t nPro
 static void fill_config(frb::InsertConfig &cfg, const fr_settings &s)
 {
   cfg.fast = s.type == FR_TYPE_FAST;
-  cfg.mode = s.interpolation == FR_INTERPOLATION_LOOKUP ? 0 : (s.alpha <= 15.f ? 1 : 3);
+  cfg.mode = s.interpolation == FR_INTERPOLATION_LOOKUP ? 0 : (s.alpha <= 15.f ? 1 : 2);
   const int taps = int(std::floor(2.f * s.blob_radius)) + 1;
   cfg.taps = taps <= 4 ? 4 : 8;
   cfg.storage = s.storage;
@@ -892,7 +891,7 @@ int fr_batch_init(fr_handle *h, const fr_batch_limits *lim, const fr_settings *s
   const size_t oItems = take(size_t(itemsCap) * frb::kWorkItemBytes);
   const size_t oJobs = take(size_t(lim->max_jobs) * sizeof(frb::JobDesc));
   const size_t oMisc = take(64);
-  const size_t oKaiser = take(cfg.mode == 3 && !cfg.fast ? size_t(frb::kKaiserTableElems) * sizeof(float2) : 0);
+  const size_t oKaiser = take(cfg.mode == 2 && !cfg.fast ? size_t(frb::kKaiserTableElems) * sizeof(float2) : 0);
   FR_CUDA(cudaMalloc(&h->scratch, off));
   h->scratch_bytes = off;
   char *base = static_cast<char *>(h->scratch);
@@ -922,7 +921,7 @@ int fr_batch_init(fr_handle *h, const fr_batch_limits *lim, const fr_settings *s
   h->upload_done = h->upload_set_done[0];
   FR_CUDA(cudaMemsetAsync(misc, 0, 64, h->stream));
   h->kaiser_table = nullptr;
-  if (cfg.mode == 3 && !cfg.fast) {
+  if (cfg.mode == 2 && !cfg.fast) {
     h->kaiser_table = reinterpret_cast<float *>(base + oKaiser);
     FR_CUDA(frb::launch_kaiser_table(h->kaiser_table, s->blob_order, s->alpha, s->blob_radius, h->constants.cIw0,
       h->stream));
@@ -961,7 +960,6 @@ static int enqueue_batch(fr_handle *h, int nJobs, int totalSpaces, int totalBric
   set_table(P, h, table, h->blim.table_elems);
   P.lutInSmem = frb::insert_lut_in_smem(h->cfg, P.tableElems);
   P.c = h->constants;
-  P.order = s.blob_order;
   FR_CUDA(frb::launch_insert(P, h->cfg, h->grid, h->stream));
   FR_CUDA(cudaMemcpyAsync(h->host_misc, h->bb.nItems, frb::kMiscBytes, cudaMemcpyDeviceToHost, h->stream));
   return FR_OK;

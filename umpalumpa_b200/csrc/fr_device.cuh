@@ -205,64 +205,6 @@ __device__ inline double bessel_in_d(int order, double x)
   return i;
 }
 
-__device__ inline float bessel_i0_f(float x)
-{
-  float ax = fabsf(x), t;
-  if (ax < 3.75f) {
-    t = x / 3.75f;
-    t *= t;
-    return 1.f
-           + t * (3.5156229f
-                  + t * (3.0899424f
-                         + t * (1.2067492f + t * (0.2659732f + t * (0.360768e-1f + t * 0.45813e-2f)))));
-  }
-  t = 3.75f / ax;
-  return (expf(ax) * (1 / sqrtf(ax)))
-         * (0.39894228f
-            + t * (0.1328592e-1f
-                   + t * (0.225319e-2f
-                          + t * (-0.157565e-2f
-                                 + t * (0.916281e-2f
-                                        + t * (-0.2057706e-1f
-                                               + t * (0.2635537e-1f
-                                                      + t * (-0.1647633e-1f + t * 0.392377e-2f))))))));
-}
-
-__device__ inline float bessel_i1_f(float x)
-{
-  float ax = fabsf(x), r, t;
-  if (ax < 3.75f) {
-    t = x / 3.75f;
-    t *= t;
-    r = ax
-        * (0.5f
-           + t * (0.87890594f
-                  + t * (0.51498869f
-                         + t * (0.15084934f + t * (0.2658733e-1f + t * (0.301532e-2f + t * 0.32411e-3f))))));
-  } else {
-    t = 3.75f / ax;
-    r = 0.2282967e-1f + t * (-0.2895312e-1f + t * (0.1787654e-1f - t * 0.420059e-2f));
-    r = 0.39894228f
-        + t * (-0.3988024e-1f + t * (-0.362018e-2f + t * (0.163801e-2f + t * (-0.1031555e-1f + t * r))));
-    r *= (expf(ax) * (1 / sqrtf(ax)));
-  }
-  return x < 0.f ? -r : r;
-}
-
-__device__ inline float bessel_in_f(int order, float x)
-{
-  if (order == 0) return bessel_i0_f(x);
-  if (order == 1) return bessel_i1_f(x);
-  if (x == 0) return 0;
-  float im1 = bessel_i0_f(x), i = bessel_i1_f(x);
-  for (int k = 1; k < order; ++k) {
-    float nx = im1 - ((2 * k) / x) * i;
-    im1 = i;
-    i = nx;
-  }
-  return i;
-}
-
 // The dynamic blob for alpha <= 15 (fr_common_kernels.hpp:163-170: bessi0Fast(alpha sqrt(1 - d2/r^2))
 // / I0(alpha) * cIw0) for two taps at once, for the insertion's tap pairs: a polynomial of degree
 // kKaiserDegree in u = 1 - d2/r^2 by Horner's rule in packed FP32x2.  The weight is a power series
@@ -280,22 +222,6 @@ __device__ __forceinline__ float2 kaiser_poly2(float2 d2, float2 negInvR2, const
 #pragma unroll
   for (int k = kKaiserDegree - 1; k >= 0; --k) h = __ffma2_rn(h, u, c[k]);
   return h;
-}
-
-// Blob value at distance r for a blob of radius a, in the device form of the reference
-// (fr_common_kernels.hpp:129-161): the Bessel ratio is scaled by 1/I_order(alpha).
-__device__ inline float kaiser_value_f(float r, float a, float alpha, float oneOverBessi, int order)
-{
-  float rda = r / a;
-  if (!(rda <= 1.f)) return 0.f;
-  float rdas = rda * rda;
-  float arg = alpha * sqrtf(1.f - rdas);
-  if (order == 0) return bessel_i0_f(arg) * oneOverBessi;
-  float w = sqrtf(1.f - rdas);
-  if (order == 2) w = w * w;
-  if (order == 3) w = w * w * w;
-  if (order == 4) w = w * w * w * w;
-  return w * (bessel_in_f(order, arg) * oneOverBessi);
 }
 
 // ------------------------------------------------------------------------------------

@@ -44,7 +44,7 @@
 
 namespace frb {
 
-enum { kModeLut = 0, kModeFastKaiser = 1, kModeKaiser = 2, kModeKaiserTable = 3 };
+enum { kModeLut = 0, kModeKaiserPoly = 1, kModeKaiserTable = 2 };
 
 // A brick's voxel (x, y, z) has the linear index 256 z + 16 y + x; its accumulators sit at that
 // index with the low five bits -- the shared-memory bank -- rotated by 5 (y / 2) + 6 z, so that
@@ -270,10 +270,8 @@ __device__ __forceinline__ bool voxel_blob(const InsertParams &P, const JobGeom 
         const int li = GENERIC ? min(int(pos), P.tableElems - 1) : int(pos);
         const float2 e = reinterpret_cast<const float2 *>(lut)[li];
         wb = fmaf(e.y, pos - float(li), e.x);
-      } else if (MODE == kModeFastKaiser) {
-        wb = pos;  // the pair's weights, computed below with kaiser_poly2
       } else {
-        wb = kaiser_value_f(sqrtf(d2), r, c.cBlobAlpha, c.cOneOverBessiOrderAlpha, P.order) * c.cIw0;
+        wb = pos;  // the pair's weights, computed below with kaiser_poly2
       }
       const float2 v = Pixel<STORAGE>::load(row + (BANDED ? 4 * jj : jj));
       w += wb;
@@ -289,11 +287,10 @@ __device__ __forceinline__ bool voxel_blob(const InsertParams &P, const JobGeom 
 #pragma unroll
     for (int k = 0; k < TAPS / 2; ++k) {
       const float2 d2 = __ffma2_rn(dxp[k], dxp[k], yz2);
-      // per tap: the table position (lookup), the blob weight (fast Kaiser) or d2
-      const float2 pos = MODE == kModeLut            ? __ffma2_rn(d2, cI2, half2)
+      // per tap: the table position, or the polynomial's blob weight
+      const float2 pos = MODE == kModeLut           ? __ffma2_rn(d2, cI2, half2)
                          : MODE == kModeKaiserTable ? __fmul2_rn(d2, kt2)
-                         : MODE == kModeFastKaiser  ? kaiser_poly2(d2, negInvR2, P.kaiser)
-                                                    : d2;
+                                                    : kaiser_poly2(d2, negInvR2, P.kaiser);
       tap(row, ii, 2 * k, d2.x, pos.x);
       tap(row, ii, 2 * k + 1, d2.y, pos.y);
     }
@@ -611,7 +608,8 @@ __global__ void __launch_bounds__(kThreads *Groups<KAHAN, FAST>::value, 1) inser
       if (FAST)
         insert_nearest<STORAGE, KAHAN, JOBS, BANDED>(P, G, A, ox, oy, oz, dir, warp, lane, e0, e1);
       else
-        insert_blobs<MODE, TAPS, STORAGE, KAHAN, JOBS, BANDED>(P, G, A, lut, sVoxels[threadIdx.x >> 5], ox, oy, oz, dir, warp, lane, e0, e1);
+        insert_blobs<MODE, TAPS, STORAGE, KAHAN, JOBS, BANDED>(P, G, A, lut, sVoxels[threadIdx.x >> 5], ox, oy, oz, dir,
+          warp, lane, e0, e1);
       group_sync(group);  // the next direction maps warps to other voxels
     }
     // add the brick into the caller's volume -- Kahan: a cut brick into its FP64 sums, which the
@@ -697,9 +695,8 @@ static InsertFn pick_mode(const InsertConfig &cfg)
   if (cfg.fast) return insert_kernel<kModeLut, 4, true, STORAGE, KAHAN, JOBS, BANDED>;
   switch (cfg.mode) {
   case kModeLut: return pick_taps<kModeLut, false, STORAGE, KAHAN, JOBS, BANDED>(cfg.taps);
-  case kModeFastKaiser: return pick_taps<kModeFastKaiser, false, STORAGE, KAHAN, JOBS, BANDED>(cfg.taps);
-  case kModeKaiserTable: return pick_taps<kModeKaiserTable, false, STORAGE, KAHAN, JOBS, BANDED>(cfg.taps);
-  default: return pick_taps<kModeKaiser, false, STORAGE, KAHAN, JOBS, BANDED>(cfg.taps);
+  case kModeKaiserPoly: return pick_taps<kModeKaiserPoly, false, STORAGE, KAHAN, JOBS, BANDED>(cfg.taps);
+  default: return pick_taps<kModeKaiserTable, false, STORAGE, KAHAN, JOBS, BANDED>(cfg.taps);
   }
 }
 

@@ -703,7 +703,7 @@ static size_t table_bytes(const InsertConfig &cfg, int tableElems)
 {
   if (cfg.fast) return 0;
   if (cfg.mode == 0) return tableElems <= kLutSmemMax ? size_t(tableElems) * sizeof(float) : 0;
-  if (cfg.mode == 3) return size_t(kKaiserTableElems) * sizeof(float2);
+  if (cfg.mode == 2) return size_t(kKaiserTableElems) * sizeof(float2);
   return 0;
 }
 

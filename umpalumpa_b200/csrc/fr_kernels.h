@@ -91,7 +91,6 @@ struct InsertParams {
   int genericTaps;  // bounds-checked taps with a clamped table index: half-plane narrower or
                     // shorter than the blob window, or a blob table above kLutSmemMax entries
   fr_constants c;
-  int order;
   int nProj;
   int fftX, fftY;
   int vx, vy, vz;
@@ -102,8 +101,8 @@ struct InsertParams {
 
 // Which insertion kernel variant runs.
 struct InsertConfig {
-  int mode;     // 0 lookup table, 1 fast Kaiser (alpha <= 15), 2 Kaiser of any order per tap,
-                // 3 Kaiser of any order from the interpolated (value, slope) table (alpha > 15)
+  int mode;     // 0 lookup table, 1 the blob's polynomial (alpha <= 15), 2 Kaiser of any order from
+                // the interpolated (value, slope) table (alpha > 15)
   int taps;     // blob footprint per axis: floor(2 r) + 1
   bool fast;    // nearest-pixel insertion (Settings::Type::kFast)
   int storage;  // FR_STORAGE_*

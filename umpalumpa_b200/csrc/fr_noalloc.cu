@@ -144,8 +144,8 @@ extern "C" int fr_insert_noalloc(int device, void *stream, const fr_dims *d, con
   cfg.fast = s->type == FR_TYPE_FAST;
   // the kernel modes of fr_execute: above alpha 15 the interpolated Kaiser table, built in
   // the scratch array by every call
-  cfg.mode = s->interpolation == FR_INTERPOLATION_LOOKUP ? 0 : (s->alpha <= 15.f ? 1 : 3);
-  const bool kaiserTable = cfg.mode == 3 && !cfg.fast;
+  cfg.mode = s->interpolation == FR_INTERPOLATION_LOOKUP ? 0 : (s->alpha <= 15.f ? 1 : 2);
+  const bool kaiserTable = cfg.mode == 2 && !cfg.fast;
   cfg.taps = int(std::floor(2.f * s->blob_radius)) + 1 <= 4 ? 4 : 8;
   cfg.storage = s->storage;
   cfg.kahan = s->accumulation == FR_ACCUM_KAHAN;
@@ -261,7 +261,6 @@ extern "C" int fr_insert_noalloc(int device, void *stream, const fr_dims *d, con
   frb::kaiser_polynomial(c.cBlobAlpha, c.cOneOverBessiOrderAlpha * c.cIw0, P.kaiser);
   P.genericTaps = int(d->fft_x) < cfg.taps || int(d->fft_y) < cfg.taps || P.tableElems > frb::kLutSmemMax;
   P.c = c;
-  P.order = s->blob_order;
   P.nProj = int(nProj);
   P.fftX = int(d->fft_x);
   P.fftY = int(d->fft_y);
