@@ -202,16 +202,6 @@ __device__ __forceinline__ bool voxel_blob(const InsertParams &P, const JobGeom 
   const float qy = add_(qy0, float(G.cy));
   const float rSq = mul_(r, r);
   const float zSq = mul_(qz, qz);
-  // Outside the frequency sphere (integer-valued: exact), behind the image or off the slab, as
-  // the reference rejects; and beyond the image's other edges, where no pixel lies within the
-  // radius (which also rejects non-finite coordinates).  One predicate: the tests are independent.
-  // The last three cost 0.3-1.1 % where no voxel lies out there (box 256 x 20,000 36.3 -> 36.4 ms),
-  // but keep a voxel that can only add zeros out of the taps -- 2,000 half-planes cropped to
-  // 33 x 64 into box 256 take 1.77 ms with them, 2.84 without -- and out of the sums, where the
-  // zeros times an infinite or NaN weight would be NaN.
-  const bool inside = !(px * px + py * py + pz * pz > s.maxDist2) & !(qx < -r) & !(zSq > rSq)
-                      & (qx <= float(G.fftX) + r) & (qy >= -r) & (qy <= float(G.fftY) + r);
-  if (!inside) return false;
   // The TAPS x TAPS window starts at (ceil(qx - r), ceil(qy - r)) shifted into the image, so
   // it covers the reference's clamped blob box [max(ceil(q - r), 0), min(floor(q + r), X-1)]
   // and lies inside the image; candidates outside the blob box have d2 > r^2, so d2 <= r^2
@@ -225,10 +215,26 @@ __device__ __forceinline__ bool voxel_blob(const InsertParams &P, const JobGeom 
     x0 = fminf(x0, float(G.fftX - TAPS));
     y0 = fminf(y0, float(G.fftY - TAPS));
   }
+  const float dx0 = sub_(qx, x0);
+  // Outside the frequency sphere (integer-valued: exact), behind the image or off the slab, as
+  // the reference rejects; and beyond the image's other edges, where no pixel lies within the
+  // radius (which also rejects non-finite coordinates).  One predicate: the tests are independent.
+  // The last three cost 0.3-0.9 % where no voxel lies out there (box 256 x 20,000 36.3 -> 36.5 ms),
+  // but keep a voxel that can only add zeros out of the taps -- 2,000 half-planes cropped to
+  // 33 x 64 into box 256 take 1.77 ms with them, 2.84 without -- and out of the sums, where the
+  // zeros times an infinite or NaN weight would be NaN.  Either form is sound where the window is
+  // shifted into the image; from the window's outer pixels, whose distances the taps use, is the faster
+  // one beside the polynomial (box 256 x 6,000 12.49 -> 12.35 ms, box 96 FP16 x 777 383 -> 380 us),
+  // from the image's size beside the table lookups (36.66 -> 36.54 ms).
+  bool inside = !(px * px + py * py + pz * pz > s.maxDist2) & !(qx < -r) & !(zSq > rSq);
+  if (GENERIC || MODE == kModeLut)
+    inside = inside & (qx <= float(G.fftX) + r) & (qy >= -r) & (qy <= float(G.fftY) + r);
+  else
+    inside = inside & (dx0 - float(TAPS - 1) <= r) & (sub_(qy, y0) >= -r) & (sub_(qy, add_(y0, float(TAPS - 1))) <= r);
+  if (!inside) return false;
   const int minX = int(x0), minY = int(y0);
   const int maxX = min(int(floorf(add_(qx, r))), G.fftX - 1);  // GENERIC only
   const int maxY = min(int(floorf(add_(qy, r))), G.fftY - 1);
-  const float dx0 = sub_(qx, x0);
   // First pixel of window row ii.  Banded: rows o = minY % 4, o + 1, ... of the window's first
   // band; row ii lies (o + ii) / 4 bands further (at most one for 4 rows), where the same row
   // offset less 4 applies.
