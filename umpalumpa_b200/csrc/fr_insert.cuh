@@ -25,11 +25,11 @@
 // beyond __syncwarp; a group synchronises (named barrier) only when the direction changes.
 //
 // What bounds it (lookup, FP32, banded, 1,537-20,000 projections at box 256): the L1/shared data
-// path (117 wavefronts per step of 32 voxels: 60 pixel gathers, 34 table lookups, 13 accumulators)
-// at 79 % and instruction issue at 66 %, with the 24 warps that shared memory and registers
-// allow.  Against steps that start anew for every projection (26 of 32 lanes filled, the source
+// path (117 wavefronts per step of 32 voxels: 60 pixels and records; 34 table lookups, 13 accumulators
+// and the lists, shuffles and flushes) at 80 % and instruction issue at 69 %, with the 24 warps that
+// shared memory and registers allow.  Against steps that start anew for every projection (26 of 32 lanes filled, the source
 // columns found by a binary search over shuffles), with one voxel body per direction instead of
-// one for all: 17 % fewer instructions and 14 % fewer wavefronts; 20,000 projections
+// one for all: 18 % fewer instructions and 14 % fewer wavefronts; 20,000 projections
 // 45.8 -> 36.3 ms (the whole call).
 //
 // Half-plane layouts (BANDED): the caller's row-major half-planes, or the same pixels in bands

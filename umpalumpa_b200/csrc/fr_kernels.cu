@@ -631,9 +631,9 @@ cudaError_t launch_binning(const BinGeom &g, const fr_traverse_space *spaces, in
   return cudaGetLastError();
 }
 
-// The band copy, the binning and the insertion all ask for the largest shared-memory carve-out,
-// so that an SM running copy CTAs (which need no shared memory) can take binning CTAs beside
-// them instead of waiting for the copy to end.
+// The band copy and the binning ask for the largest shared-memory carve-out, so that an SM running
+// copy CTAs (which need no shared memory) can take binning CTAs beside them instead of waiting for
+// the copy to end.  The insertion's shared memory leaves no smaller one to choose.
 template<typename K> static void prefer_max_shared(K *kernel)
 {
   if (cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared)
