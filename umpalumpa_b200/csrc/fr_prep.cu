@@ -175,7 +175,7 @@ struct fr_prep {
 namespace {
 
 // Side of the fused route for these settings (0: cuFFT route).  It is the faster one at every side
-// and storage it covers, few images or many (fr_prep_fft.cuh; kSplit has the one exception).
+// and storage it covers, few images or many (fr_prep_fft.cuh, kSplit).
 int fused_side(const fr_prep_settings &s)
 {
   if (s.fft == FR_PREP_FFT_CUFFT || s.size_x != s.size_y) return 0;
