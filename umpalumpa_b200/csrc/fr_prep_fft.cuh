@@ -225,12 +225,13 @@ template<int N> struct Shape {
 };
 
 // CTAs an image is split between in a call of few images: FP32 sides from 192 on, where one CTA per
-// image is slower than cuFFT up to 4 (192), 8 (256) or 12 images (320, 384).  It is the latency of the passes' N / 32 rounds,
-// which the CTAs of a cluster share: 1, 8, 32 and 37 images of side 320 take 19, 19, 21 and 33 us
-// (one CTA each 51; cuFFT 43, 48, 64 and 68), of side 384 21, 21, 23 and 41 (70; 56, 62, 86 and 88).
-// Side 256: 1, 32 and 74 images 12, 13 and 25 us (35; 29, 38 and 45), side 192: 1, 32 and 111 images 11, 12
-// and 22 us (25; 23, 27 and 41).  At the smaller sides, and with 16-bit output, one CTA per image is
-// faster than cuFFT at every number of images (side 128: 14.5 against 16.5; BF16 side 384: 92 against 106).
+// image is slower than cuFFT up to 2 (192), 8 (256) or 12 images (320, 384).  It is the latency of the
+// passes' N / 32 rounds, which the CTAs of a cluster share: 1, 8, 32 and 37 images of side 320 take 19,
+// 19, 21 and 33 us (one CTA each 51; cuFFT 43, 48, 64 and 68), of side 384 21, 21, 23 and 41 (70; 56,
+// 62, 86 and 88); 1, 32 and 74 of side 256 12, 13 and 25 (35; 29, 38 and 45); 1, 32 and 111 of side 192
+// 11, 12 and 22 (25 to 27; 23, 27 and 41).  At the smaller sides, and with 16-bit output, one CTA per
+// image is faster than cuFFT at every number of images (side 128 14.5 against 16.5 us, BF16 side 384 92
+// against 106).
 constexpr int kSplit = 4;
 template<int N, int STORAGE> constexpr bool kSplits = N >= 192 && STORAGE == FR_STORAGE_FP32;
 
