@@ -189,7 +189,7 @@ __device__ __forceinline__ float voxel_coord(int i, float origin) { return __int
 // gather of the projection pixels within the blob radius.  The blob weights are summed raw
 // and scaled by the space weight (and the storage scale) once at the end.  Returns false if
 // the voxel is rejected.
-template<int MODE, int TAPS, int STORAGE, bool GENERIC, bool BANDED>
+template<int MODE, int TAPS, int STORAGE, bool GENERIC, bool JOBS, bool BANDED>
 __device__ __forceinline__ bool voxel_blob(const InsertParams &P, const JobGeom &G, const VoxelRec &s,
   const typename Pixel<STORAGE>::T *__restrict__ img, int bandStride, float scale, const float *lut, float px,
   float py, float pz, float2 &ov, float &ow)
@@ -227,7 +227,7 @@ __device__ __forceinline__ bool voxel_blob(const InsertParams &P, const JobGeom 
   // one beside the polynomial (box 256 x 6,000 12.49 -> 12.35 ms, box 96 FP16 x 777 383 -> 380 us),
   // from the image's size beside the table lookups (36.66 -> 36.54 ms).
   bool inside = !(px * px + py * py + pz * pz > s.maxDist2) & !(qx < -r) & !(zSq > rSq);
-  if (GENERIC || MODE == kModeLut)
+  if (GENERIC || (MODE == kModeLut && !JOBS))
     inside = inside & (qx <= float(G.fftX) + r) & (qy >= -r) & (qy <= float(G.fftY) + r);
   else
     inside = inside & (dx0 - float(TAPS - 1) <= r) & (sub_(qy, y0) >= -r) & (sub_(qy, add_(y0, float(TAPS - 1))) <= r);
@@ -470,9 +470,9 @@ __device__ __forceinline__ void insert_blobs(const InsertParams &P, const JobGeo
       const float scale = STORAGE == FR_STORAGE_FP32 ? 1.f : __ldg(G.scales + s.proj);
       const PT *img = reinterpret_cast<const PT *>(G.fft) + size_t(unsigned(s.proj)) * plane;
       if (G.genericTaps)
-        ok = voxel_blob<MODE, TAPS, STORAGE, true, BANDED>(P, G, s, img, bandStride, scale, lut, px, py, pz, v, w);
+        ok = voxel_blob<MODE, TAPS, STORAGE, true, JOBS, BANDED>(P, G, s, img, bandStride, scale, lut, px, py, pz, v, w);
       else
-        ok = voxel_blob<MODE, TAPS, STORAGE, false, BANDED>(P, G, s, img, bandStride, scale, lut, px, py, pz, v, w);
+        ok = voxel_blob<MODE, TAPS, STORAGE, false, JOBS, BANDED>(P, G, s, img, bandStride, scale, lut, px, py, pz, v, w);
     }
     const int slot = acc_slot(voxel & 4095);
     if (parts == 1) {  // two steps of three
