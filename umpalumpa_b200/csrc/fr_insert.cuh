@@ -224,8 +224,10 @@ __device__ __forceinline__ bool voxel_blob(const InsertParams &P, const JobGeom 
   // 33 x 64 into box 256 take 1.77 ms with them, 2.84 without -- and out of the sums, where the
   // zeros times an infinite or NaN weight would be NaN.  Either form is sound where the window is
   // shifted into the image; from the window's outer pixels, whose distances the taps use, is the faster
-  // one beside the polynomial (box 256 x 6,000 12.49 -> 12.35 ms, box 96 FP16 x 777 383 -> 380 us),
-  // from the image's size beside the table lookups (36.66 -> 36.54 ms).
+  // one beside the polynomial (box 256 x 6,000 12.49 -> 12.35 ms, box 96 FP16 x 777 383 -> 380 us) and
+  // in batched launches, whose image size lies in shared memory (against the kernel without the tests,
+  // six streamed jobs 0.992x -> 1.000x, twelve captured jobs 0.998x -> 1.003x); from the image's size
+  // beside the table lookups of a single job (36.66 -> 36.54 ms).
   bool inside = !(px * px + py * py + pz * pz > s.maxDist2) & !(qx < -r) & !(zSq > rSq);
   if (GENERIC || (MODE == kModeLut && !JOBS))
     inside = inside & (qx <= float(G.fftX) + r) & (qy >= -r) & (qy <= float(G.fftY) + r);
